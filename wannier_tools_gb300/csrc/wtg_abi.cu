@@ -929,7 +929,7 @@ static int unit_op(int op, int n, const double* a, const double* b, double* c, i
   cudaError_t e = cudaMemcpy(dx, a, sizeof(double2) * nn, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && op == 0) e = cudaMemcpy(dy, b, sizeof(double2) * nn, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
-    e = mixed ? wtg::launch_mixed_unit(op, n, dx, dy, dc, dws, 8, dst, 0)
+    e = mixed ? wtg::launch_mixed_unit(op, n, dx, 8, dst, 0)
               : wtg::launch_fp64_unit(op, n, dx, dy, dc, dws, dst, 0);
   if (e == cudaSuccess) e = cudaMemcpy(c, dc, sizeof(double2) * nn, cudaMemcpyDeviceToHost);
   int st = 0;

@@ -232,9 +232,8 @@ cudaError_t launch_batch_mixed(const BatchArgs& a, const DecimConfig& cfg, int g
 size_t batch_ws_matrices(int precision_mixed);
 
 // One product (op 0: C = X*Y) or inverse (op 1: C = X^-1) by a single CTA.
-// Mixed: ws holds 5 N x N complex matrices; FP64: work holds two.
-cudaError_t launch_mixed_unit(int op, int N, const double2* X, const double2* Y, double2* C,
-                              double2* ws, int ns, int* status, cudaStream_t s);
+// Mixed: W holds X, Y, C and five work matrices; FP64: work holds two matrices.
+cudaError_t launch_mixed_unit(int op, int N, double2* W, int ns, int* status, cudaStream_t s);
 cudaError_t launch_fp64_unit(int op, int N, const double2* X, const double2* Y, double2* C,
                              double2* work, int* status, cudaStream_t s);
 
