@@ -57,8 +57,13 @@ extern "C" {
                                    the point's outputs are not valid */
 
 /* precision modes */
-#define WTG_PREC_FP64  0        /* all-FP64 decimation (FP64 DFMA pipe); Ndim <= 320 (above
-                                   119 the inverse runs in global memory) */
+#define WTG_PREC_FP64  0        /* FP64 decimation; Ndim <= 320.  At Ndim 33..256 every product is
+                                   an exactly split product on the tcgen05 tensor cores (55-bit
+                                   operands in balanced 8-bit digits, exact integer accumulation,
+                                   smaller error than an FP64 product) and an inverse an FP32
+                                   Gauss-Jordan refined on such products to FP64's residual, or
+                                   the FP64 Gauss-Jordan where that does not converge (condition
+                                   beyond ~1e7); at other Ndim all on the FP64 pipe */
 #define WTG_PREC_MIXED 1        /* products as BF16 digit splits on the tcgen05 tensor cores
                                    (49-bit rounded operands in balanced 7-bit digits, FP32
                                    accumulation exact per slice order up to 6, int64
@@ -368,10 +373,10 @@ int wtg_batch_spectrum(int nmodels, const wtg_model_t* models, int npts, const i
  * Test-only switches, process-wide (no counterpart in the reference).  They
  * exist so that a test can reach code paths that normal inputs do not; a
  * production caller never sets them.  value 0 restores normal operation.
- *   WTG_TEST_FP64_GLOBAL_INVERSE  non-zero: the per-model FP64 kernel inverts in
- *                                 global memory at every Ndim (the variant that
- *                                 normally runs above Ndim 119; both agree bit
- *                                 for bit)
+ *   WTG_TEST_FP64_GLOBAL_INVERSE  non-zero: the per-model FP64 kernels' FP64
+ *                                 Gauss-Jordan runs in global memory at every
+ *                                 Ndim (the variant for large matrices; both
+ *                                 agree bit for bit)
  *   WTG_TEST_MIXED_SPIN_LIMIT     > 0: the mixed kernels' pipeline waits on the
  *                                 tensor cores give up after this many
  *                                 non-blocking polls instead of the built-in

@@ -382,7 +382,7 @@ int engine_create(int nmodels, const wtg_model_t* models, int precision, int max
     if (ce == cudaSuccess) ce = wtg::batch_mixed_config(max_n, &e->wb, &e->cfg);
   } else {
     ce = wtg::batch_fp64_prepare();
-    if (ce == cudaSuccess) ce = wtg::batch_fp64_config(max_n, ph_bytes, &e->smem_gj_max, &e->cfg);
+    if (ce == cudaSuccess) ce = wtg::batch_fp64_config(max_n, ph_bytes, &e->smem_gj_max, &e->wb, &e->cfg);
   }
   if (ce != cudaSuccess) {
     delete e;
@@ -398,7 +398,7 @@ int engine_create(int nmodels, const wtg_model_t* models, int precision, int max
     return fail(WTG_EUNSUPPORTED, "batch kernel shared memory exceeds the device limit");
   }
   e->grid = nsm * std::max(1, e->cfg.ctas_per_sm);
-  e->ws_stride = wtg::batch_ws_matrices(mixed ? 1 : 0) * (size_t)max_n * max_n;
+  e->ws_stride = wtg::batch_ws_matrices(e->cfg) * (size_t)max_n * max_n;
   // device tables
   std::vector<int> lists;
   size_t ot = 0, ob = 0;
@@ -778,7 +778,7 @@ int wtg_surfgreen_1985(int ndim, double omega, double eta, const double* h00, co
   const size_t nn = (size_t)ndim * ndim;
   wtg::DecimConfig cfg;
   WTG_CK(wtg::decim_fp64_config(ndim, 0, &cfg));
-  // one allocation: h[2nn] | gll grr gb [3nn] | ws [8 or 9 nn] | omega | outputs
+  // one allocation: h[2nn] | gll grr gb [3nn] | ws [8, 9 or 11 nn] | omega | outputs
   const size_t wsm = wtg::decim_fp64_ws_matrices(cfg);
   const size_t bytes = sizeof(double2) * ((5 + wsm) * nn) + 64 + 64;
   char* base = nullptr;
@@ -930,7 +930,7 @@ static int unit_op(int op, int n, const double* a, const double* b, double* c, i
   if (e == cudaSuccess && op == 0) e = cudaMemcpy(dy, b, sizeof(double2) * nn, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = mixed ? wtg::launch_mixed_unit(op, n, dx, 8, dst, 0)
-              : wtg::launch_fp64_unit(op, n, dx, dy, dc, dws, dst, 0);
+              : wtg::launch_fp64_unit(op, n, dx, dst, 0);
   if (e == cudaSuccess) e = cudaMemcpy(c, dc, sizeof(double2) * nn, cudaMemcpyDeviceToHost);
   int st = 0;
   if (e == cudaSuccess) e = cudaMemcpy(&st, dst, sizeof(int), cudaMemcpyDeviceToHost);

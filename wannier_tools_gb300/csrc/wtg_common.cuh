@@ -166,8 +166,8 @@ struct BatchArgs {
   size_t ws_stride;           // double2 per CTA
   int* counter;               // zero at launch
   int KC;                     // FP64 GEMM k-chunk
-  int smem_gj_max;            // FP64: largest Ndim whose inverse runs in shared memory
-  int wb;                     // mixed: B-plane width of the shared-memory layout
+  int smem_gj_max;            // FP64 pipe kernel: largest Ndim whose inverse runs in shared memory
+  int wb;                     // split products: B-plane width of the shared-memory layout
   size_t ph_off;              // byte offset of the phase table (max nRu double2) in shared memory
 };
 
@@ -179,6 +179,7 @@ struct DecimConfig {
   int ctas_per_sm;
   int inv_global = 0;         // FP64: 1 = the inverse runs in global memory (large Ndim)
   int w0 = 0;                 // mixed: output-column pass width
+  int split = 0;              // products on the tensor cores (mixed form; FP64 form's split kernel)
 };
 
 // Built-in choices and limits of the tunable shapes, and the mixed form's pass
@@ -221,21 +222,39 @@ cudaError_t decim_mixed_config(int N, DecimConfig* cfg);
 cudaError_t launch_decimate_mixed(const DecimArgs& a, const DecimConfig& cfg, int grid,
                                   cudaStream_t s);
 
+// The FP64 form on exactly split tensor-core products (wtg_split64.cu) runs in
+// this range of Ndim.  Below it a product fills too little of a 128-row tile.
+// Above it the form stays on the FP64 pipe: its results there (Ndim 264, eta
+// 1e-3 eV) are compared to 1e-9 with FP64 evaluations that are themselves up to
+// 2e-9 off (80-bit evaluation of the same points; the split kernel is within
+// 2e-10 of it, the FP64 pipe within 9e-10), so only the plain operations agree
+// with them everywhere.
+constexpr int FP64_SPLIT_MIN_N = 33;
+constexpr int FP64_SPLIT_MAX_N = 256;
+constexpr bool fp64_split(int N) { return N >= FP64_SPLIT_MIN_N && N <= FP64_SPLIT_MAX_N; }
+cudaError_t split64_config(int N, DecimConfig* cfg);
+cudaError_t launch_split64(const DecimArgs& a, const DecimConfig& cfg, int grid, cudaStream_t s);
+cudaError_t batch_split64_config(int max_n, int* wb, DecimConfig* cfg);
+cudaError_t batch_split64_prepare();
+cudaError_t launch_batch_split64(const BatchArgs& a, const DecimConfig& cfg, int grid,
+                                 cudaStream_t s);
+
 // Uneven batch launch shapes and launches.  The configs' shared memory excludes the
 // phase table, which the caller appends at BatchArgs::ph_off and adds to cfg.smem before
 // launching; extra_smem reserves room for it.
-cudaError_t batch_fp64_config(int max_n, size_t extra_smem, int* smem_gj_max, DecimConfig* cfg);
+cudaError_t batch_fp64_config(int max_n, size_t extra_smem, int* smem_gj_max, int* wb,
+                              DecimConfig* cfg);
 cudaError_t launch_batch_fp64(const BatchArgs& a, const DecimConfig& cfg, int grid, cudaStream_t s);
 cudaError_t batch_mixed_config(int max_n, int* wb, DecimConfig* cfg);
 cudaError_t launch_batch_mixed(const BatchArgs& a, const DecimConfig& cfg, int grid, cudaStream_t s);
 // Workspace matrices per CTA of the batch kernels.
-size_t batch_ws_matrices(int precision_mixed);
+size_t batch_ws_matrices(const DecimConfig& cfg);
 
-// One product (op 0: C = X*Y) or inverse (op 1: C = X^-1) by a single CTA.
-// Mixed: W holds X, Y, C and five work matrices; FP64: work holds two matrices.
+// One product (op 0: C = X*Y) or inverse (op 1: C = X^-1) by a single CTA: W
+// holds X, Y, C and five work matrices.
 cudaError_t launch_mixed_unit(int op, int N, double2* W, int ns, int* status, cudaStream_t s);
-cudaError_t launch_fp64_unit(int op, int N, const double2* X, const double2* Y, double2* C,
-                             double2* work, int* status, cudaStream_t s);
+cudaError_t launch_fp64_unit(int op, int N, double2* W, int* status, cudaStream_t s);
+cudaError_t launch_split64_unit(int op, int N, double2* W, int* status, cudaStream_t s);
 
 // Sets the calling thread's message returned by wtg_last_error.
 void set_last_error(const char* msg);

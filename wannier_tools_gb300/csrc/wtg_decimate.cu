@@ -33,158 +33,7 @@ namespace {
 
 #include "wtg_fp64_dev.cuh"
 
-// Options of one solve for the batch kernel, with the member names of
-// DecimArgs (whose kernel parameter the plain kernel passes directly, so its
-// lists are read from parameter space).  Orbital lists are 1-based.
-struct SolveOpts {
-  int nw;
-  double tol;
-  int itermax;
-  int divide_by_pi;
-  int ntop, nbot;
-  const int* top;
-  const int* bot;
-  double* spin[6];             // null: no spin-resolved sums
-  int spin_right_bottom;
-};
-
-// The products of one decimation step.  At the large Ndim of the global-memory
-// inverse the eight workspaces of all resident CTAs no longer fit the L2, so
-// operands come from DRAM and their staging is double-buffered.
-template <int RP, int EPI, bool GI>
-__device__ __forceinline__ double gemm(const double2* X, const double2* Y, int N, int KC,
-                                       const Shared& s, double2* out0, double2* out1) {
-  if (GI) return cta_gemm_db<RP, EPI>(X, Y, N, KC, s.sX, out0, out1);
-  return cta_gemm<RP, EPI>(X, Y, N, KC, s.sX, s.sY, out0, out1);
-}
-
-// Decimation of one instance whose eps, eps_s, eps_t (= H00), alpha (= H01)
-// and beta (= H01^dagger) already sit in workspace matrices 0..4 of W; the
-// spectral sums of the three final inverses are handed to emit(dl, dr, db,
-// spin[6], iterations, status) in thread 0, the inverses themselves go to
-// gll / grr / gb when those are not null.
-// GI = false: the inverse runs in shared memory (Ndim <= decim_fp64_max_n());
-// GI = true: it runs in workspace matrix 8 in global memory, in panels
-// (gj_invert_global; Ndim <= 320).
-template <int RP, bool GI, class O, class Emit>
-__device__ void fp64_solve(int N, int KC, double2 w, const O& o, double2* gll, double2* grr,
-                           double2* gb, double2* W, const Shared& s, Emit emit) {
-  const int NN = N * N, tid = threadIdx.x;
-  double2* Mg = GI ? W + (size_t)8 * NN : nullptr;   // global-memory inverse work
-  double2* E = W;
-  double2* ES = W + (size_t)NN;
-  double2* ET = W + (size_t)2 * NN;
-  double2* Al = W + (size_t)3 * NN;
-  double2* Be = W + (size_t)4 * NN;
-  double2* G = W + (size_t)5 * NN;
-  double2* M1 = W + (size_t)6 * NN;
-  double2* M2 = W + (size_t)7 * NN;
-  // (w - X)^-1, optionally stored un-permuted to dst; ginv reads the result
-  // blk 1 / 2: only the leading / trailing Num_wann block of the inverse (one
-  // principal layer), from the Schur complement of the rest, where the spectral
-  // sums read nothing else (schur_block_invert); a zero pivot there takes the
-  // full inverse.  With GI the block's inverse needs its Num_wann^2 area within
-  // the stage area every launch of this Ndim has (KC = 16).
-  const int m = N - o.nw;
-  const bool gblk = !GI || schur_area_bytes(N, o.nw) <= fp64_gi_smem_bytes(N);
-  const Shared fb = schur_layout(reinterpret_cast<unsigned char*>(s.big), N, o.nw);
-  int blk = 0;
-  auto invert = [&](const double2* X, double2* dst, int want_blk) -> int {
-    blk = (gblk && !dst && m > 0) ? want_blk : 0;
-    if (blk && !(GI ? schur_block_invert_global(X, w, N, o.nw, blk == 1, Mg, fb)
-                    : schur_block_invert(X, w, N, o.nw, blk == 1, s)))
-      return 0;
-    blk = 0;
-    int sing;
-    if (GI) {
-      sing = gj_invert_global(X, w, N, Mg, s);
-      if (dst) gj_store_global(N, Mg, s, dst);
-    } else {
-      sing = gj_invert(X, w, N, s);
-      if (dst) gj_store(N, s, dst);
-    }
-    return sing;
-  };
-  auto ginv = [&](int i, int j) {
-    if (blk) {                        // block entry (i, j): local indices in the block
-      const int li = blk == 1 ? o.nw - 1 - i : i - m;
-      const int lj = blk == 1 ? o.nw - 1 - j : j - m;
-      return GI ? fb.big[li + (size_t)fb.cols[lj] * o.nw]
-                : s.big[m + li + (size_t)(m + s.cols[lj]) * N];
-    }
-    return GI ? Mg[i + (size_t)s.cols[j] * N] : s.big[i + s.cols[j] * N];
-  };
-
-  int st = 0, it = 0;
-  bool conv = false;
-  for (int itc = 1; itc <= o.itermax; ++itc) {                // src/surfgreen.f90:86
-    it = itc;
-    if (invert(E, G, 0)) st |= PT_SINGULAR;                   // :88-89
-    __syncthreads();
-    gemm<RP, EPI_STORE, GI>(Al, G, N, KC, s, M1, nullptr);              // :92
-    gemm<RP, EPI_STORE, GI>(Be, G, N, KC, s, M2, nullptr);              // :95
-    gemm<RP, EPI_ADD2, GI>(M1, Be, N, KC, s, E, ES);                    // :98-102
-    gemm<RP, EPI_ADD2, GI>(M2, Al, N, KC, s, E, ET);                    // :107-110
-    double part = gemm<RP, EPI_STORE_NORM, GI>(M1, Al, N, KC, s, G, nullptr);  // :113
-    gemm<RP, EPI_STORE, GI>(M2, Be, N, KC, s, M1, nullptr);             // :116
-    // rotate buffers: alpha <- G, beta <- M1
-    double2* t0 = Al;
-    Al = G;
-    G = t0;
-    double2* t1 = Be;
-    Be = M1;
-    M1 = t1;
-    const double nrm = block_sum(part, s);                    // :120
-    if (nrm <= o.tol) {                                       // :121
-      conv = true;
-      break;
-    }
-  }
-  if (!conv) st |= PT_NOT_CONVERGED;
-
-  double dl = 0.0, dr = 0.0, db = 0.0;
-  double spin[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  // GLL = (w - eps_s)^-1                                     // :127-128
-  if (invert(ES, gll, 1)) st |= PT_SINGULAR;
-  if (tid == 0) {
-    for (int q = 0; q < o.ntop; ++q) {
-      const int io = o.top[q] - 1;
-      const double v = ginv(io, io).y;
-      dl = o.divide_by_pi ? dl - v / PI_REF : dl - v;
-    }
-    if (o.spin[0])                                            // src/surfstat.f90:162-177
-      spin_sums(ginv, o.nw, o.ntop, o.top, 0, o.divide_by_pi, spin[0], spin[1], spin[2]);
-  }
-  __syncthreads();
-  // GRR = (w - eps_t)^-1                                     // :130-131
-  // surfstat's spin sums read GRR's leading block as well (src/surfstat.f90:178-192)
-  if (invert(ET, grr, (o.spin[0] && !o.spin_right_bottom) ? 0 : 2)) st |= PT_SINGULAR;
-  if (tid == 0) {
-    for (int q = 0; q < o.nbot; ++q) {
-      const int io = N - o.nw + o.bot[q] - 1;
-      const double v = ginv(io, io).y;
-      dr = o.divide_by_pi ? dr - v / PI_REF : dr - v;
-    }
-    if (o.spin[0]) {                                          // src/surfstat.f90:178-192
-      if (o.spin_right_bottom)                                // src/fermiarc.f90:300-327
-        spin_sums(ginv, o.nw, o.nbot, o.bot, N - o.nw, o.divide_by_pi, spin[3], spin[4], spin[5]);
-      else
-        spin_sums(ginv, o.nw, o.ntop, o.top, 0, o.divide_by_pi, spin[3], spin[4], spin[5]);
-    }
-  }
-  __syncthreads();
-  // GB = (w - eps)^-1                                        // :133-134
-  if (invert(E, gb, 0)) st |= PT_SINGULAR;
-  if (tid == 0) {
-    for (int i = 0; i < N; ++i) {
-      const double v = ginv(i, i).y;
-      db = o.divide_by_pi ? db - v / PI_REF : db - v;
-    }
-    if (!isfinite(dl) || !isfinite(dr) || !isfinite(db)) st |= PT_NONFINITE;
-    emit(dl, dr, db, spin, it, st);
-  }
-  __syncthreads();
-}
+#include "wtg_fp64_solve.cuh"
 
 template <int RP, bool GI>
 __global__ void __launch_bounds__(GI ? 256 : 512, 1) k_decimate_fp64(const __grid_constant__ DecimArgs a) {
@@ -281,30 +130,23 @@ __global__ void __launch_bounds__(256, 1) k_batch_fp64(const __grid_constant__ B
   }
 }
 
-// one product C = X*Y (op 0) or inverse C = X^-1 (op 1) in FP64 by one CTA;
-// gi: the inverse in global memory (work: negX then Mg, N x N each)
-template <bool GI>
-__global__ void __launch_bounds__(GI ? 256 : 512, 1) k_fp64_unit(int op, int N, int KC,
-                                                     const double2* X, const double2* Y,
-                                                     double2* C, double2* negX, double2* Mg,
-                                                     int* status) {
+// one product (op 0) or inverse (op 1) on the FP64 pipe by one CTA (Ndim below
+// FP64_SPLIT_MIN_N): W holds X, Y, the result and work matrices
+__global__ void __launch_bounds__(512, 1) k_fp64_unit(int op, int N, int KC, double2* W,
+                                                      int* status) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int NN = N * N;
-  const Shared s = fp64_layout(smraw, N, KC, !GI);
+  const Shared s = fp64_layout(smraw, N, KC, true);
+  double2* const C = W + 2 * NN;
   if (op == 0) {
-    cta_gemm<13, EPI_STORE>(X, Y, N, KC, s.sX, s.sY, C, nullptr);
+    cta_gemm<13, EPI_STORE>(W, W + NN, N, KC, s.sX, s.sY, C, nullptr);
     if (threadIdx.x == 0) *status = 0;
   } else {
-    for (int e = threadIdx.x; e < NN; e += blockDim.x) negX[e] = make_double2(-X[e].x, -X[e].y);
+    double2* const negX = W + 3 * NN;
+    for (int e = threadIdx.x; e < NN; e += blockDim.x) negX[e] = make_double2(-W[e].x, -W[e].y);
     __syncthreads();
-    int sing;
-    if (GI) {                                                   // (0 I - (-X))^-1
-      sing = gj_invert_global(negX, make_double2(0.0, 0.0), N, Mg, s);
-      gj_store_global(N, Mg, s, C);
-    } else {
-      sing = gj_invert(negX, make_double2(0.0, 0.0), N, s);
-      gj_store(N, s, C);
-    }
+    const int sing = gj_invert(negX, make_double2(0.0, 0.0), N, s);   // (0 I - (-X))^-1
+    gj_store(N, s, C);
     if (threadIdx.x == 0) *status = sing ? PT_SINGULAR : 0;
   }
 }
@@ -332,9 +174,12 @@ int decim_fp64_large_max_n() { return 32 * GJ_ROWS; }
 
 int fp64_threads_default(int N) { return N <= 48 ? 128 : (N <= 80 ? 256 : 512); }
 
-size_t decim_fp64_ws_matrices(const DecimConfig& cfg) { return cfg.inv_global ? 9 : 8; }
+size_t decim_fp64_ws_matrices(const DecimConfig& cfg) {
+  return cfg.split ? 11 : cfg.inv_global ? 9 : 8;
+}
 
-cudaError_t decim_fp64_config(int N, int threads_override, DecimConfig* cfg, bool force_global) {
+// launch shape of the kernel on the FP64 pipe
+static cudaError_t dfma_config(int N, int threads_override, DecimConfig* cfg, bool force_global) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -373,8 +218,18 @@ cudaError_t decim_fp64_config(int N, int threads_override, DecimConfig* cfg, boo
   return cudaSuccess;
 }
 
+cudaError_t decim_fp64_config(int N, int threads_override, DecimConfig* cfg, bool force_global) {
+  if (fp64_split(N)) {
+    const cudaError_t e = split64_config(N, cfg);
+    cfg->inv_global = force_global ? 1 : 0;       // of the FP64 fallback inverse
+    return e;
+  }
+  return dfma_config(N, threads_override, cfg, force_global);
+}
+
 cudaError_t launch_decimate_fp64(const DecimArgs& a, const DecimConfig& cfg, int grid,
                                  cudaStream_t s) {
+  if (cfg.split) return launch_split64(a, cfg, grid, s);
   if (cfg.inv_global) {
     k_decimate_fp64<13, true><<<grid, cfg.threads, cfg.smem, s>>>(a);
     return cudaGetLastError();
@@ -387,7 +242,7 @@ cudaError_t launch_decimate_fp64(const DecimArgs& a, const DecimConfig& cfg, int
   return cudaGetLastError();
 }
 
-size_t batch_ws_matrices(int precision_mixed) { return precision_mixed ? 11 : 9; }
+size_t batch_ws_matrices(const DecimConfig& cfg) { return cfg.split ? 11 : 9; }
 
 static size_t batch_fp64_smem(int max_n, int max_smem_gj_n, int KC) {
   size_t b = smem_bytes(max_n, KC, false);
@@ -398,7 +253,12 @@ static size_t batch_fp64_smem(int max_n, int max_smem_gj_n, int KC) {
   return b;
 }
 
-cudaError_t batch_fp64_config(int max_n, size_t extra_smem, int* smem_gj_max, DecimConfig* cfg) {
+cudaError_t batch_fp64_config(int max_n, size_t extra_smem, int* smem_gj_max, int* wb,
+                              DecimConfig* cfg) {
+  if (max_n >= FP64_SPLIT_MIN_N) {
+    *smem_gj_max = 0;
+    return batch_split64_config(max_n, wb, cfg);
+  }
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -438,28 +298,25 @@ cudaError_t batch_fp64_prepare() {
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(k_batch_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                optin - (int)fa.sharedSizeBytes);
+  if (err == cudaSuccess) err = batch_split64_prepare();
   if (err == cudaSuccess && dev < 64) done[dev] = true;
   return err;
 }
 
 cudaError_t launch_batch_fp64(const BatchArgs& a, const DecimConfig& cfg, int grid, cudaStream_t s) {
+  if (cfg.split) return launch_batch_split64(a, cfg, grid, s);
   k_batch_fp64<<<grid, cfg.threads, cfg.smem, s>>>(a);
   return cudaGetLastError();
 }
 
-cudaError_t launch_fp64_unit(int op, int N, const double2* X, const double2* Y, double2* C,
-                             double2* work, int* status, cudaStream_t st) {
+cudaError_t launch_fp64_unit(int op, int N, double2* W, int* status, cudaStream_t st) {
+  if (N >= FP64_SPLIT_MIN_N) return launch_split64_unit(op, N, W, status, st);
   DecimConfig cfg;
-  cudaError_t e = decim_fp64_config(N, 512, &cfg);
+  cudaError_t e = dfma_config(N, 512, &cfg, false);
   if (e != cudaSuccess) return e;
-  const void* fn = cfg.inv_global ? (const void*)k_fp64_unit<true> : (const void*)k_fp64_unit<false>;
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem);
+  e = cudaFuncSetAttribute(k_fp64_unit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem);
   if (e != cudaSuccess) return e;
-  double2* mg = work + (size_t)N * N;
-  if (cfg.inv_global)
-    k_fp64_unit<true><<<1, cfg.threads, cfg.smem, st>>>(op, N, cfg.KC, X, Y, C, work, mg, status);
-  else
-    k_fp64_unit<false><<<1, 512, cfg.smem, st>>>(op, N, cfg.KC, X, Y, C, work, mg, status);
+  k_fp64_unit<<<1, 512, cfg.smem, st>>>(op, N, cfg.KC, W, status);
   return cudaGetLastError();
 }
 

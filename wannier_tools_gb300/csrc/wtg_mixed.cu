@@ -387,6 +387,7 @@ cudaError_t decim_mixed_config(int N, DecimConfig* cfg) {
   cfg->threads = MX_T;
   cfg->KC = 0;
   cfg->RP = 0;
+  cfg->split = 1;
   cfg->w0 = mx_plan(N, tile_value(1, N)).w0;
   // at least 116 KB so that two CTAs never share an SM (each allocates all 512 TMEM columns)
   const size_t sm = mixed_smem(N, cfg->w0);
@@ -421,6 +422,7 @@ cudaError_t batch_mixed_config(int max_n, int* wb, DecimConfig* cfg) {
     smem = smem > t ? smem : t;
   }
   *wb = w;
+  cfg->split = 1;
   cfg->threads = MX_T;
   cfg->KC = 0;
   cfg->RP = 0;

@@ -6,8 +6,8 @@
 // fragments the pool), and latency-critical loops in which cudaMalloc /
 // cudaFree would synchronise the whole device and stall work on other
 // streams.  For them, wtg_surfgreen_batch_noalloc runs the FP64 decimation
-// kernel with its scratch (the per-CTA workspace of eight Ndim x Ndim complex
-// matrices and the work counter) taken from the fixed array below instead of
+// kernel with its scratch (the per-CTA workspace of Ndim x Ndim complex
+// matrices, eleven or eight by Ndim, and the work counter) taken from the fixed array below instead of
 // from device allocations.  The caller passes every input and output as device
 // memory it already owns.
 //
@@ -81,12 +81,6 @@ extern "C" int wtg_surfgreen_batch_noalloc(int ndim, int nw, int nk, const doubl
   if (ndim > wtg::decim_fp64_max_n())
     return nerr(WTG_EUNSUPPORTED, "ndim " + std::to_string(ndim) + " exceeds the kernel limit " +
                                       std::to_string(wtg::decim_fp64_max_n()));
-  const size_t per_cta = sizeof(double2) * 8 * (size_t)ndim * ndim;
-  const size_t counter_bytes = 256;
-  if (per_cta + counter_bytes > WTG_NOALLOC_SCRATCH_BYTES)
-    return nerr(WTG_EUNSUPPORTED, "one CTA's workspace (" + std::to_string(per_cta) +
-                                      " bytes) exceeds the fixed scratch of " +
-                                      std::to_string(WTG_NOALLOC_SCRATCH_BYTES) + " bytes");
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices)
@@ -100,6 +94,12 @@ extern "C" int wtg_surfgreen_batch_noalloc(int ndim, int nw, int nk, const doubl
   e = wtg::decim_fp64_config(ndim, 0, &cfg);
   if (e != cudaSuccess) return nerr(WTG_ECUDA, std::string("config: ") + cudaGetErrorString(e));
   if (cfg.ctas_per_sm < 1) return nerr(WTG_EUNSUPPORTED, "decimation kernel does not fit an SM");
+  const size_t per_cta = sizeof(double2) * wtg::decim_fp64_ws_matrices(cfg) * (size_t)ndim * ndim;
+  const size_t counter_bytes = 256;
+  if (per_cta + counter_bytes > WTG_NOALLOC_SCRATCH_BYTES)
+    return nerr(WTG_EUNSUPPORTED, "one CTA's workspace (" + std::to_string(per_cta) +
+                                      " bytes) exceeds the fixed scratch of " +
+                                      std::to_string(WTG_NOALLOC_SCRATCH_BYTES) + " bytes");
   int nsm = 0;
   e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return nerr(WTG_ECUDA, cudaGetErrorString(e));

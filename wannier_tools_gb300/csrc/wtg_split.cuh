@@ -219,6 +219,7 @@ struct DigB7 {
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
   static constexpr int KSPLIT = 1 << 20;              // K of one exact accumulation
   static constexpr bool POISON = false;
+  static constexpr bool FRO = false;
   static constexpr int SLOT = D == 7 ? 0 : 2;         // its issue tables (full and last width)
 
   static constexpr unsigned long long BIAS =
@@ -315,6 +316,7 @@ struct DigF8 {
   static constexpr uint32_t IDESC = (1u << 4) | ((128u >> 4) << 24);
   static constexpr int KSPLIT = 160;
   static constexpr int SLOT = D == 7 ? 0 : 2;
+  static constexpr bool FRO = true;
   static constexpr bool POISON = true;                // Inf / NaN in a row or column give NaN
 
   static constexpr unsigned long long BIAS = 0x80808080808080ull;
@@ -852,8 +854,11 @@ __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, 
             val = make_double2(old0[jj].x + val.x, old0[jj].y + val.y);
           }
           o0b[(size_t)j * N] = val;
-          if ((epi == OZ_STORE_NORM || epi == OZ_IMINUS) && last)
-            nrm += fabsf(d2f_bits(val.x)) + fabsf(d2f_bits(val.y));
+          if ((epi == OZ_STORE_NORM || epi == OZ_IMINUS) && last) {
+            const float fr = d2f_bits(val.x), fi = d2f_bits(val.y);
+            if (K::FRO && epi == OZ_IMINUS) nrm = fmaf(fr, fr, fmaf(fi, fi, nrm));
+            else nrm += fabsf(fr) + fabsf(fi);
+          }
           e = max(bexp(val.x), bexp(val.y));
         }
         rmax = max(rmax, e);
@@ -877,7 +882,7 @@ __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, 
 // (the first product's last, partly filled tile takes its first rows; each
 // output element sees the same digits and sums as in a product of its own).
 // Returns this thread's FP32 partial of a sum over the outputs: OZ_STORE_NORM
-// and OZ_IMINUS sum |re| + |im|.
+// and OZ_IMINUS sum |re| + |im| (OZ_IMINUS of a kind with FRO: re^2 + im^2).
 template <class K>
 __device__ __noinline__ float split_gemm(double2* __restrict__ const W, const uint32_t op,
                                          const int EPI, const int EPI2, const int N, const int NP,

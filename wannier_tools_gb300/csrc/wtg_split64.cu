@@ -1,0 +1,452 @@
+// FP64 Lopez-Sancho decimation with its products on the 5th-generation tensor
+// cores (Ndim FP64_SPLIT_MIN_N .. FP64_SPLIT_MAX_N; other sizes run in
+// wtg_decimate.cu).
+//
+// GB300 issues two FP64 FMAs a clock per SM: the FP64 pipe at 91-95 % was the
+// bound of the whole form, 20 M cycles an iteration at Ndim 112.  Here every
+// complex product of surfgreen_1985 (src/surfgreen.f90:92-116, zgemm at
+// src/mat_mul.f90:23) is an exactly split product (split_gemm of wtg_split.cuh
+// with DigF8 digits): 55-bit operands against a shared exponent per row /
+// column, seven base-256 digits, the slice orders 2..9 in one exact integer
+// accumulator each.  Its error (operand rounding, 2^-55 of the row or column
+// maximum) is below that of an FP64 product, whose partial sums round K times:
+// against exact products of normal random complex matrices it is 3-6 times
+// smaller at Ndim 40..320.
+//
+// Inverses (zgesv with identity, src/inverse.f90:43-55): an FP32 Gauss-Jordan
+// with partial pivoting gives a starting point, and Newton-Schulz steps
+// X <- X + X (I - M X) with the residual as a split product are taken until
+// |I - M X|_F <= 1e-8 before a step, so that the step leaves its square, below
+// the residual's own rounding: an FP64 inverse with a right residual as small
+// as a pivoted elimination's.  Where the residual does not get there (condition
+// beyond ~1e7, an FP32 zero pivot, infinities), the FP64 Gauss-Jordan of the
+// plain form runs instead, with its singular flag.
+#include <mutex>
+
+#include "../../include/wtgpu.h"
+#include "wtg_common.cuh"
+
+namespace wtg {
+
+namespace {
+
+#include "wtg_fp64_dev.cuh"
+#include "wtg_split.cuh"
+#include "wtg_fp64_solve.cuh"
+
+using Dig7 = DigF8<7>;
+using Dig4 = DigF8<4>;
+
+__host__ __device__ inline MxPlan s64_plan(int N) { return split_plan(N, split_wmax<Dig7>()); }
+
+__device__ __forceinline__ float gemm7(double2* W, uint32_t op, int epi, int epi2, const MxPlan& p,
+                                       const MxShared s) {
+  return split_gemm<Dig7>(W, op, epi, epi2, p.N, p.NP, p.w0, p.ncb, s);
+}
+__device__ __forceinline__ void gemm4(double2* W, uint32_t op, int epi, const MxPlan& p7,
+                                      const MxShared s) {
+  const MxPlan p = split_plan4(p7);
+  split_gemm<Dig4>(W, op, epi, -1, p.N, p.NP, p.w0, p.ncb, s);
+}
+
+// the FP64 Gauss-Jordan of the plain form, un-permuted into dst; its area
+// aliases the stages and the exponents.  Mg: work for the global-memory variant.
+__device__ __noinline__ int gj64(const double2* X, double2 w, int N, double2* dst, double2* Mg,
+                                 int gi) {
+  extern __shared__ __align__(1024) unsigned char smem_dyn[];
+  const bool gsm = N <= MX_SMEM_GJ_N && !gi;
+  const Shared fs = fp64_layout(smem_dyn, N, GJ_PANEL, gsm);
+  __syncthreads();
+  int sing;
+  if (gsm) {
+    sing = gj_invert(X, w, N, fs);
+    gj_store(N, fs, dst);
+  } else {
+    sing = gj_invert_global(X, w, N, Mg, fs);
+    gj_store_global(N, Mg, fs, dst);
+  }
+  __syncthreads();
+  return sing;
+}
+
+// (w I - W[iX])^-1 into workspace matrix G with its exponents (see the head of
+// the file).  Uses matrices Mi, R, Gn as work; swaps G and Gn.  live0 / live1:
+// matrices whose exponents a fallback has to make again (-1: none).
+__device__ int s64_inverse(int iX, double2 w, double2* W, const MxPlan& pl, int& G, int& Gn, int Mi,
+                           int R, int live0, int live1, int gi, const MxShared s) {
+  const int N = pl.N;
+  const size_t NN = (size_t)N * N;
+  bool good = false;
+  if (!gj32(W + iX * NN, w, N, W, Mi, G, R, s)) {
+    float prev = 3.0e38f;
+    for (int t = 0; t < 8 && !s.t().abort; ++t) {
+      // R = I - M G; the sum is |R|_F^2
+      const float res = sqrtf(block_sum_f(gemm7(W, ops(Mi, G, R), OZ_IMINUS, -1, pl, s), s));
+      if (!(res < 0.25f * prev)) break;               // no longer converging (or NaN)
+      // Gn = G + G R: 30 bits of R keep the step's own error below |R| 2^-30
+      gemm4(W, ops(G, R, Gn, G), OZ_ADDTO, pl, s);
+      swap_mat(G, Gn);
+      if (res <= 1e-8f) {                             // the step left at most 1e-16
+        good = true;
+        break;
+      }
+      prev = res;
+    }
+  }
+  if (good || s.t().abort) return 0;
+  const int sing = gj64(W + iX * NN, w, N, W + G * NN, W + Mi * NN, gi);
+  exps_of(W + G * NN, G, N, s);
+  if (live0 >= 0) exps_of(W + live0 * NN, live0, N, s);
+  if (live1 >= 0) exps_of(W + live1 * NN, live1, N, s);
+  return sing;
+}
+
+// sum over q = 0 .. n-1 of f(q), subtracted term by term in order (as the
+// reference's loops), the terms evaluated by all threads; result in thread 0
+template <class F>
+__device__ double list_sum(int n, F f, const MxShared s) {
+  double* buf = reinterpret_cast<double*>(s.base());
+  constexpr int NB = 4096;
+  double acc = 0.0;
+  for (int q0 = 0; q0 < n; q0 += NB) {
+    const int m = min(NB, n - q0);
+    __syncthreads();
+    for (int q = threadIdx.x; q < m; q += blockDim.x) buf[q] = f(q0 + q);
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int q = 0; q < m; ++q) acc = acc - buf[q];
+  }
+  __syncthreads();
+  return acc;
+}
+
+// spin terms of orbital io (1-based list entry + offset - 1): see spin_sums
+__device__ __forceinline__ double spin_term(const double2* G, int N, int nw, int io, int c) {
+  const int nwh = nw / 2, jl = io % nw;
+  int partner = -1;
+  double sgn = 0.0;
+  if (jl < nwh) {
+    partner = io + nwh;
+    sgn = 1.0;
+  } else if (jl < 2 * nwh) {
+    partner = io - nwh;
+    sgn = -1.0;
+  }
+  if (partner < 0) return 0.0;
+  if (c == 2) return sgn * G[io + (size_t)io * N].y;
+  const double2 gp = G[io + (size_t)partner * N];
+  return c == 0 ? gp.y : sgn * gp.x;
+}
+
+// Decimation of one instance whose eps, eps_s, eps_t (= H00), alpha (= H01) and
+// beta (= H01^dagger) already sit in workspace matrices 0..4 of W (11 N x N
+// matrices), as fp64_solve; all threads.
+template <class O, class Emit>
+__device__ __forceinline__ void s64_solve(const MxPlan& pl, double2 w, const O& o, double2* gll,
+                                          double2* grr, double2* gb, double2* W, int gi,
+                                          const MxShared s, Emit emit) {
+  const int N = pl.N, NN = N * N, tid = threadIdx.x;
+  int Al = 3, Be = 4, G = 5, R = 9, Gn = 10;          // workspace matrices by index
+  constexpr int iE = 0, iES = 1, iET = 2, M1 = 6, M2 = 7, iMi = 8;
+  int stat = 0, it = 0;
+  bool conv = false;
+  split_tables<Dig7, Dig4>(pl, s);
+  exps_of(W + (size_t)Al * NN, Al, N, s);
+  exps_dagger(Be, Al, N, s);
+  for (int itc = 1; itc <= o.itermax && !s.t().abort; ++itc) {   // src/surfgreen.f90:86-122
+    it = itc;
+    if (s64_inverse(iE, w, W, pl, G, Gn, iMi, R, Al, Be, gi, s)) stat |= PT_SINGULAR;
+    // the six products (:92-116), row-stacked where that takes fewer 128-row
+    // tiles; eps still receives M1 beta before M2 alpha
+    float part;
+    if ((2 * N + 127) / 128 < 2 * ((N + 127) / 128)) {
+      gemm7(W, ops(Al, G, M1, 0, Be, M2), OZ_STORE, OZ_STORE, pl, s);               // :92, :95
+      gemm7(W, ops(M1, Be, iE, iES, M2, R), OZ_ADD2, OZ_STORE, pl, s);              // :98-102, :116
+      part = gemm7(W, ops(M1, Al, Gn, 0, M2, iE, iET), OZ_STORE_NORM, OZ_ADD2, pl, s);  // :113, :107-110
+    } else {
+      gemm7(W, ops(Al, G, M1), OZ_STORE, -1, pl, s);                                // :92
+      gemm7(W, ops(Be, G, M2), OZ_STORE, -1, pl, s);                                // :95
+      gemm7(W, ops(M1, Be, iE, iES), OZ_ADD2, -1, pl, s);                           // :98-102
+      part = gemm7(W, ops(M1, Al, Gn), OZ_STORE_NORM, -1, pl, s);                   // :113
+      gemm7(W, ops(M2, Al, iE, iET), OZ_ADD2, -1, pl, s);                           // :107-110
+      gemm7(W, ops(M2, Be, R), OZ_STORE, -1, pl, s);                                // :116
+    }
+    swap_mat(Al, Gn);
+    swap_mat(Be, R);
+    if (converged(part, W + (size_t)Al * NN, N, o.tol, s)) {     // :120-122
+      conv = true;
+      break;
+    }
+  }
+  if (!conv) stat |= PT_NOT_CONVERGED;
+
+  // GLL = (w - eps_s)^-1, GRR = (w - eps_t)^-1, GB = (w - eps)^-1   // :127-134
+  double sums[9];                                   // dl, dr, db, then the six spin sums
+  for (int k = 0; k < 3; ++k) {
+    const int iX = k == 0 ? iES : k == 1 ? iET : iE;
+    double2* const dst = k == 0 ? gll : k == 1 ? grr : gb;
+    if (s64_inverse(iX, w, W, pl, G, Gn, iMi, R, -1, -1, gi, s)) stat |= PT_SINGULAR;
+    __syncthreads();
+    const double2* const g = W + (size_t)G * NN;
+    if (dst)
+      for (int e = tid; e < NN; e += blockDim.x) dst[e] = g[e];
+    const int n = k == 0 ? o.ntop : k == 1 ? o.nbot : N;
+    auto idx = [&](int q) {
+      return k == 0 ? o.top[q] - 1 : k == 1 ? N - o.nw + o.bot[q] - 1 : q;
+    };
+    auto scaled = [&](double v) { return o.divide_by_pi ? v / PI_REF : v; };
+    sums[k] = list_sum(n, [&](int q) {
+      const int io = idx(q);
+      return scaled(g[io + (size_t)io * N].y);
+    }, s);
+    if (k < 2 && o.spin[0]) {                       // src/surfstat.f90:162-192
+      // surfstat's right sums run over the top list (as the reference's do)
+      const bool top = k == 0 || !o.spin_right_bottom;
+      const int off = top ? 0 : N - o.nw;
+      for (int c = 0; c < 3; ++c)
+        sums[3 + 3 * k + c] = list_sum(top ? o.ntop : o.nbot, [&](int q) {
+          return scaled(spin_term(g, N, o.nw, off + (top ? o.top[q] : o.bot[q]) - 1, c));
+        }, s);
+    }
+  }
+  if (tid == 0) {
+    if (s.t().abort) stat |= PT_TIMEOUT;
+    if (!isfinite(sums[0]) || !isfinite(sums[1]) || !isfinite(sums[2])) stat |= PT_NONFINITE;
+    emit(sums[0], sums[1], sums[2], sums + 3, it, stat);
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(SP_T, 1) k_decimate_split64(const __grid_constant__ DecimArgs a,
+                                                              int gi) {
+  const int N = a.N, NN = N * N, T = blockDim.x, tid = threadIdx.x;
+  const MxPlan pl = s64_plan(N);
+  const MxShared s = mx_layout(pl.wb);
+  mx_setup(s, 0u);
+  double2* W = a.ws + (size_t)blockIdx.x * 11 * NN;
+  for (;;) {
+    if (tid == 0) s.t().misc[0] = atomicAdd(a.counter, 1);
+    __syncthreads();
+    const int inst = s.t().misc[0];
+    __syncthreads();
+    if (inst >= a.n_inst) break;
+    const int ik = inst / a.nomega, iw = inst % a.nomega;
+    const size_t oidx = (size_t)(a.k_offset + ik) + (size_t)iw * a.nk_total;
+    if (s.t().abort) {       // a wait gave up earlier: the rest of this CTA's points are not computed
+      if (tid == 0) {
+        const double nan = __longlong_as_double(0x7FF8000000000000LL);
+        a.dos_l[oidx] = nan;
+        a.dos_r[oidx] = nan;
+        a.dos_bulk[oidx] = nan;
+        if (a.spin[0])
+          for (int c = 0; c < 6; ++c) a.spin[c][oidx] = nan;
+        if (a.iters) a.iters[oidx] = 0;
+        if (a.status) a.status[oidx] = (uint8_t)PT_TIMEOUT;
+      }
+      continue;
+    }
+    const double2* H00 = a.h + (size_t)ik * 2 * NN;
+    const double2* H01 = H00 + NN;
+    const double2 w = make_double2(a.omega[iw], a.eta);      // src/surfgreen.f90:82
+    for (int e = tid; e < NN; e += T) {                       // :74-78
+      const double2 h = H00[e];
+      W[e] = h;
+      W[NN + e] = h;
+      W[2 * NN + e] = h;
+      const double2 t = H01[e];
+      W[3 * NN + e] = t;
+      const int i = e % N, j = e / N;
+      W[4 * NN + j + (size_t)i * N] = make_double2(t.x, -t.y);
+    }
+    __syncthreads();
+    s64_solve(pl, w, a, a.gll ? a.gll + (size_t)inst * NN : nullptr,
+              a.grr ? a.grr + (size_t)inst * NN : nullptr,
+              a.gb ? a.gb + (size_t)inst * NN : nullptr, W, gi, s,
+              [&](double dl, double dr, double db, const double* spin, int it, int stat) {
+                a.dos_l[oidx] = dl;
+                a.dos_r[oidx] = dr;
+                a.dos_bulk[oidx] = db;
+                if (a.spin[0])
+                  for (int c = 0; c < 6; ++c) a.spin[c][oidx] = spin[c];
+                if (a.iters) a.iters[oidx] = it;
+                if (a.status) a.status[oidx] = (uint8_t)stat;
+              });
+  }
+  mx_teardown(s);
+}
+
+// Uneven batch (several models, eta per point) in one persistent launch, as
+// k_batch_fp64 of wtg_decimate.cu: points outside the split range run on the FP64
+// pipe, the others as k_decimate_split64.
+__global__ void __launch_bounds__(SP_T, 1) k_batch_split64(const __grid_constant__ BatchArgs a) {
+  extern __shared__ __align__(1024) unsigned char smem_dyn[];
+  const int tid = threadIdx.x;
+  const MxShared s = mx_layout(a.wb);
+  mx_setup(s, 0u);
+  double2* W = a.ws + (size_t)blockIdx.x * a.ws_stride;
+  const int npts = a.run ? a.run->npts : a.npts;
+  const double tol = a.run ? a.run->tol : a.tol;
+  const int itermax = a.run ? a.run->itermax : a.itermax;
+  const int divide_by_pi = a.run ? a.run->divide_by_pi : a.divide_by_pi;
+  for (;;) {
+    if (tid == 0) {
+      const int q = atomicAdd(a.counter, 1);
+      s.t().misc[0] = q < npts ? a.order[q] : -1;
+    }
+    __syncthreads();
+    const int p = s.t().misc[0];
+    __syncthreads();
+    if (p < 0) break;
+    if (s.t().abort) {                // a wait gave up earlier: not computed
+      if (tid == 0) {
+        const double nan = __longlong_as_double(0x7FF8000000000000LL);
+        a.dos_l[p] = nan;
+        a.dos_r[p] = nan;
+        a.dos_bulk[p] = nan;
+        if (a.iters) a.iters[p] = 0;
+        if (a.status) a.status[p] = PT_TIMEOUT;
+      }
+      continue;
+    }
+    const BatchModel& m = a.models[a.pmodel[p]];
+    fourier_fill(m, a.k[p], a.k[p + a.npts], W, reinterpret_cast<double2*>(smem_dyn + a.ph_off));
+    SolveOpts o;
+    o.nw = m.nw;
+    o.tol = tol;
+    o.itermax = itermax;
+    o.divide_by_pi = divide_by_pi;
+    o.ntop = m.ntop;
+    o.nbot = m.nbot;
+    o.top = m.top;
+    o.bot = m.bot;
+    for (int c = 0; c < 6; ++c) o.spin[c] = nullptr;
+    o.spin_right_bottom = 0;
+    const double2 w = make_double2(a.omega[p], a.eta[p]);
+    auto emit = [&](double dl, double dr, double db, const double*, int it, int st) {
+      a.dos_l[p] = dl;
+      a.dos_r[p] = dr;
+      a.dos_bulk[p] = db;
+      if (a.iters) a.iters[p] = it;
+      if (a.status) a.status[p] = (uint8_t)st;
+    };
+    constexpr int KC = 16;
+    if (m.N > FP64_SPLIT_MAX_N) {
+      fp64_solve<13, true>(m.N, KC, w, o, nullptr, nullptr, nullptr, W,
+                           fp64_layout(smem_dyn, m.N, KC, false), emit);
+    } else if (m.N < FP64_SPLIT_MIN_N) {
+      fp64_solve<13, false>(m.N, KC, w, o, nullptr, nullptr, nullptr, W,
+                            fp64_layout(smem_dyn, m.N, KC, true), emit);
+    } else {
+      MxPlan pl = s64_plan(m.N);
+      pl.wb = a.wb;
+      s64_solve(pl, w, o, nullptr, nullptr, nullptr, W, 0, s, emit);
+    }
+  }
+  mx_teardown(s);
+}
+
+// one product (op 0) or inverse (op 1) by one CTA: W holds X, Y, the result and
+// five work matrices
+__global__ void __launch_bounds__(SP_T, 1) k_split64_unit(int op, int N, double2* W, int* status) {
+  const MxPlan pl = s64_plan(N);
+  const int NN = N * N, tid = threadIdx.x;
+  const MxShared s = mx_layout(pl.wb);
+  mx_setup(s, 0u);
+  split_tables<Dig7, Dig4>(pl, s);
+  int sing = 0;
+  if (op == 0) {
+    exps_of(W, 0, N, s);
+    exps_of(W + NN, 1, N, s);
+    gemm7(W, ops(0, 1, 2), OZ_STORE, -1, pl, s);
+  } else {
+    // C = X^-1: X given directly, so pass -X with w = 0 (M = 0*I - (-X) = X)
+    double2* negX = W + 7 * (size_t)NN;
+    for (int e = tid; e < NN; e += blockDim.x) negX[e] = make_double2(-W[e].x, -W[e].y);
+    __syncthreads();
+    int G = 3, Gn = 4;
+    sing = s64_inverse(7, make_double2(0.0, 0.0), W, pl, G, Gn, 5, 6, -1, -1, 0, s);
+    __syncthreads();
+    double2* C = W + 2 * (size_t)NN;
+    for (int e = tid; e < NN; e += blockDim.x) C[e] = W[(size_t)G * NN + e];
+  }
+  if (tid == 0) *status = (s.t().abort ? PT_TIMEOUT : 0) | (sing ? PT_SINGULAR : 0);
+  mx_teardown(s);
+}
+
+static_assert(fp64_gi_smem_bytes(MX_MAXN) <= MX_FP64_AREA, "the FP64 pipe's stages fit the area");
+
+size_t s64_smem(int wb) {
+  // at least 116 KB so that two CTAs never share an SM (each allocates all 512 TMEM columns)
+  const size_t b = split_smem(wb);
+  return b > (size_t)(116 << 10) ? b : (size_t)(116 << 10);
+}
+
+}  // namespace
+
+cudaError_t split64_config(int N, DecimConfig* cfg) {
+  if (N > MX_MAXN) return cudaErrorInvalidValue;
+  cfg->threads = SP_T;
+  cfg->KC = 0;
+  cfg->RP = 0;
+  cfg->split = 1;
+  cfg->smem = s64_smem(s64_plan(N).wb);
+  cudaError_t e = cudaFuncSetAttribute(k_decimate_split64,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg->smem);
+  if (e != cudaSuccess) return e;
+  int occ = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_decimate_split64, SP_T, cfg->smem);
+  if (e != cudaSuccess) return e;
+  cfg->ctas_per_sm = occ > 1 ? 1 : occ;       // tensor memory is allocated whole (512 columns)
+  return cudaSuccess;
+}
+
+cudaError_t batch_split64_config(int max_n, int* wb, DecimConfig* cfg) {
+  if (max_n > MX_MAXN) return cudaErrorInvalidValue;
+  int w = 8;
+  for (int n = FP64_SPLIT_MIN_N; n <= max_n && n <= FP64_SPLIT_MAX_N; ++n)
+    w = w > s64_plan(n).wb ? w : s64_plan(n).wb;
+  *wb = w;
+  cfg->threads = SP_T;
+  cfg->KC = 0;
+  cfg->RP = 0;
+  cfg->split = 1;
+  cfg->smem = s64_smem(w);
+  cfg->ctas_per_sm = 1;
+  return cudaSuccess;
+}
+
+// the batch kernel's dynamic shared-memory limit raised to the opt-in maximum
+cudaError_t batch_split64_prepare() {
+  int dev = 0, optin = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  cudaFuncAttributes fa;
+  if (err == cudaSuccess)
+    err = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, k_batch_split64);
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(k_batch_split64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               optin - (int)fa.sharedSizeBytes);
+  return err;
+}
+
+cudaError_t launch_batch_split64(const BatchArgs& a, const DecimConfig& cfg, int grid,
+                                 cudaStream_t s) {
+  k_batch_split64<<<grid, cfg.threads, cfg.smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_split64_unit(int op, int N, double2* W, int* status, cudaStream_t s) {
+  const size_t smem = s64_smem(s64_plan(N).wb);
+  cudaError_t e =
+      cudaFuncSetAttribute(k_split64_unit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_split64_unit<<<1, SP_T, smem, s>>>(op, N, W, status);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_split64(const DecimArgs& a, const DecimConfig& cfg, int grid, cudaStream_t s) {
+  k_decimate_split64<<<grid, cfg.threads, cfg.smem, s>>>(a, cfg.inv_global);
+  return cudaGetLastError();
+}
+
+}  // namespace wtg
