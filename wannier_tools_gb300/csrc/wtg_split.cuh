@@ -458,11 +458,8 @@ __host__ __device__ __forceinline__ int planes_bytes_of(int WB) {
 }
 // small arrays, at their byte offsets behind that region
 struct SplitTail {
-  float2 colbuf[MX_SMEM_GJ_N];   // multiplier columns of the shared-memory FP32 Gauss-Jordan
-  float2 rowbuf[MX_SMEM_GJ_N];
   float2 recip[MX_PANEL];
-  int perm[MX_MAXN];
-  int cols[MX_MAXN];
+  int prow[MX_MAXN];             // Gauss-Jordan: pivot rows
   int pos_of[MX_MAXN];           // Gauss-Jordan: position of a row, row at a position
   int row_at[MX_MAXN];
   IssueTab tabs[4];              // a 7-digit product's full and last pass width, then a 4-digit one's
@@ -478,8 +475,9 @@ struct SplitTail {
   int misc[5];                   // 0 instance, 1 singular, 2-3 pivot rows (shared-memory Gauss-Jordan)
 };
 constexpr int SPLIT_TAIL = (int)sizeof(SplitTail);
-// the FP32 Gauss-Jordan areas fit below the exponents for every stage width
-static_assert(MX_SMEM_GJ_N * MX_SMEM_GJ_N * 8 <= 2 * 2 * MAXD * APLANE, "FP32 GJ area");
+// the FP32 Gauss-Jordan areas (matrix and multipliers) fit below the exponents for
+// every stage width
+static_assert((MX_SMEM_GJ_N + MX_PANEL) * MX_SMEM_GJ_N * 8 <= 2 * 2 * MAXD * APLANE, "FP32 GJ area");
 static_assert(MX_MAXN * MX_PANEL * 8 <= 2 * 2 * MAXD * APLANE, "FP32 GJ panel area");
 
 __host__ __device__ __forceinline__ size_t split_smem(int WB) {
@@ -1011,17 +1009,23 @@ __device__ bool converged(float part, const double2* __restrict__ Al, int N, dou
   return block_sum_d(d, s) <= tol;
 }
 
-// entry m (warp-uniform) of a 4-entry register column, without local memory
-__device__ __forceinline__ float2 pick4(const float2 (&x)[4], int m) {
-  float2 v = x[0];
-  v = m == 1 ? x[1] : v;
-  v = m == 2 ? x[2] : v;
-  v = m == 3 ? x[3] : v;
-  return v;
+// a complex float as one 64-bit register pair, for the packed FMA (two IEEE
+// FP32 FMAs in one instruction)
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
 }
-
-__device__ __forceinline__ float2 shfl_f2c(float2 v, int src) {
-  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
+                                                   unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
 
 // Gauss-Jordan without physical row swaps: row i of the working matrix stays
@@ -1029,94 +1033,152 @@ __device__ __forceinline__ float2 shfl_f2c(float2 v, int src) {
 // swapped form.  Step t's pivot is the first maximal |re| + |im| of column t
 // over the rows at positions >= t (izamax's rule in position order), so the
 // pivots, and every FMA of every entry, are those of the swapped form; only
-// the storage order differs.  Publishes the multiplier column (column t as it
-// stands), the pivot's position (perm[t]) and physical row (misc[2 + (t & 1)])
-// and its reciprocal, and moves the pivot to position t.
-__device__ __forceinline__ void gj_pivot_publish_u(const float2 (&x)[4], int t, int N, float2* cb,
-                                                float2* recip, int* perm, int* misc, int* pos_of,
-                                                int* row_at) {
+// the storage order differs.  For column t in registers (lane l of the warp
+// holds rows l + 32 m): publishes the multiplier column (column t as it stands)
+// to cb, the pivot's row to prow[t] and its reciprocal to *rslot, and moves the
+// pivot to position t.
+// Every lane prepares the reciprocal of its own best candidate while the warp
+// finds the maximum (redux.sync of the key, then of the position), and the
+// winning lane writes: the chain from the column to the published pivot has no
+// division and no shuffle.
+template <int R>
+__device__ __forceinline__ void gj_pivot_publish(const unsigned long long (&x)[R], int t, int N,
+                                                 float2* cb, float2* rslot, int* prow, int* misc,
+                                                 int* pos_of, int* row_at) {
   const int lane = threadIdx.x & 31;
-  int bkey = -1, bpos = 0x7fffffff, brow = N;
+  const int rk = row_at[t];              // moves to the pivot's position
+  int ps[R];
 #pragma unroll
-  for (int m = 0; m < 4; ++m) {
+  for (int m = 0; m < R; ++m) ps[m] = pos_of[min(lane + 32 * m, N - 1)];
+  unsigned bkey = 0;                      // key + 1; 0: no candidate
+  int bpos = 0x7fffffff, bm = 0;
+  float2 bv = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int m = 0; m < R; ++m) {
     const int i = lane + 32 * m;
-    if (i < N) {
-      const int ps = pos_of[i];
-      const int key = __float_as_int(fabsf(x[m].x) + fabsf(x[m].y));
-      if (ps >= t && (key > bkey || (key == bkey && ps < bpos))) {
-        bkey = key;
-        bpos = ps;
-        brow = i;
-      }
+    const float2 v = unpack2(x[m]);
+    if (i < N) cb[i] = v;
+    const unsigned key = (i < N && ps[m] >= t)
+                             ? (unsigned)__float_as_int(fabsf(v.x) + fabsf(v.y)) + 1u : 0u;
+    if (key > bkey || (key == bkey && key && ps[m] < bpos)) {
+      bkey = key;
+      bpos = ps[m];
+      bm = m;
+      bv = v;
     }
   }
-  {  // warp maximum of the key, then the smallest position among the lanes that hold it
-    const unsigned kmax = __reduce_max_sync(0xffffffffu, (unsigned)(bkey + 1));
-    const bool cand = (unsigned)(bkey + 1) == kmax;
-    const int pmin = (int)__reduce_min_sync(0xffffffffu, cand ? (unsigned)bpos : 0xffffffffu);
-    const int src = __ffs(__ballot_sync(0xffffffffu, cand && bpos == pmin)) - 1;
-    brow = __shfl_sync(0xffffffffu, brow, src);
-    bkey = (int)kmax - 1;
-    bpos = pmin;
-  }
-  const float2 xp = shfl_f2c(pick4(x, brow >> 5), brow & 31);
-#pragma unroll
-  for (int m = 0; m < 4; ++m) {
-    const int i = lane + 32 * m;
-    if (i < N) cb[i] = x[m];
-  }
-  if (lane == 0) {
-    perm[t] = bpos;
-    misc[2 + (t & 1)] = brow;
-    const int rk = row_at[t];            // the row at position t moves to the pivot's position
+  const float inv_d = 1.0f / __fmaf_rn(bv.x, bv.x, __fmul_rn(bv.y, bv.y));
+  const float2 rc = make_float2(bv.x * inv_d, -bv.y * inv_d);
+  const unsigned kmax = __reduce_max_sync(0xffffffffu, bkey);
+  const bool cand = bkey == kmax;
+  const unsigned pmin = __reduce_min_sync(0xffffffffu, cand ? (unsigned)bpos : 0xffffffffu);
+  if (cand && (unsigned)bpos == pmin) {   // one lane: positions are distinct
+    const int brow = lane + 32 * bm;
+    prow[t] = brow;
     row_at[bpos] = rk;
     pos_of[rk] = bpos;
     row_at[t] = brow;
     pos_of[brow] = t;
-    if (bkey == 0) {
-      misc[1] = 1;
-    } else {
-      const float inv_d = 1.0f / (xp.x * xp.x + xp.y * xp.y);
-      recip[t & 1] = make_float2(xp.x * inv_d, -xp.y * inv_d);
-    }
+    if (kmax == 1u) misc[1] = 1;
+    else *rslot = rc;
   }
 }
 
+// One Gauss-Jordan step (pivot row p, reciprocal r, multiplier column cm in
+// shared memory) applied to C columns held in registers (R rows a lane, packed),
+// rows in place; column `own` (if any) is the pivot column itself.  Per entry
+// v - f nk with the operations of four FMAs, re: -f.x nk.x, + f.y nk.y; im:
+// -f.x nk.y, - f.y nk.x, as two packed ones.  The multipliers of a step are
+// loaded once for all C columns.
+template <int R, int C, int PM>
+__device__ __forceinline__ void gj_step_at(unsigned long long (&x)[C][R],
+                                           const unsigned long long (&fa)[R],
+                                           const unsigned long long (&fb)[R], int pl, float2 r,
+                                           int own) {
+  const bool here = (threadIdx.x & 31) == pl;
+  float2 nk[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const float2 v = unpack2(x[c][PM]);
+    const float2 a = make_float2(__shfl_sync(0xffffffffu, v.x, pl), __shfl_sync(0xffffffffu, v.y, pl));
+    nk[c] = make_float2(fmaf(a.x, r.x, -a.y * r.y), fmaf(a.x, r.y, a.y * r.x));
+    if (C == 1 && c == own) {             // the pivot column becomes a column of the inverse
+      nk[c] = r;
+#pragma unroll
+      for (int m = 0; m < R; ++m) x[c][m] = 0ull;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const unsigned long long n0 = pack2(nk[c].x, nk[c].y), n1 = pack2(nk[c].y, nk[c].x);
+#pragma unroll
+    for (int m = 0; m < R; ++m) x[c][m] = fma2(fb[m], n1, fma2(fa[m], n0, x[c][m]));
+    if (here) x[c][PM] = n0;
+  }
+}
+// the row slot p / 32 of the pivot is the same for the whole warp: one branch
+// instead of R selects a column
+template <int R, int C>
+__device__ __forceinline__ void gj_step_cols(unsigned long long (&x)[C][R],
+                                             const float2* __restrict__ cm, int N, int p, float2 r,
+                                             int own) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long fa[R], fb[R];
+#pragma unroll
+  for (int m = 0; m < R; ++m) {
+    const float2 f = cm[min(lane + 32 * m, N - 1)];      // rows >= N hold nothing
+    fa[m] = pack2(-f.x, -f.x);
+    fb[m] = pack2(f.y, -f.y);
+  }
+  const int pm = p >> 5, pl = p & 31;
+#define WTG_GJ_AT(M)                                                                   \
+  if constexpr (R > M) {                                                               \
+    if (pm == M) gj_step_at<R, C, (M < R ? M : 0)>(x, fa, fb, pl, r, own);             \
+  }
+  WTG_GJ_AT(0) WTG_GJ_AT(1) WTG_GJ_AT(2) WTG_GJ_AT(3) WTG_GJ_AT(4)
+  WTG_GJ_AT(5) WTG_GJ_AT(6) WTG_GJ_AT(7) WTG_GJ_AT(8) WTG_GJ_AT(9)
+#undef WTG_GJ_AT
+}
+
 // M = w I - X (FP64, kept in Mi for the refinement, with its row exponents),
-// then FP32 Gauss-Jordan into G (FP64, with its row and column exponents).  Returns 1 on an exact zero pivot (G = identity then).
-// Ndim <= 112.  Each pivot step is one pass in which every warp takes whole
-// columns into registers (lane l holds rows l, l+32, ...): the pivot-row
-// scaling and the elimination of a column happen in registers with one
-// shuffle pair.  Rows stay in place (gj_pivot_publish_u), so an entry needs
-// one select besides its four FMAs; the output reads the rows back in pivot
-// order.  The warp that owns column k+1 also finds step k+1's pivot
-// (look-ahead) and publishes its multiplier column into the other of two
-// buffers, so a step needs one barrier.  Same operations per entry as the
-// step-by-step form with row swaps.
+// then FP32 Gauss-Jordan with partial pivoting into G (FP64, with its row and
+// column exponents).  Returns 1 on an exact zero pivot (G = identity then).
+// Ndim <= 112, the matrix in shared memory.  The pivot steps run in panels of
+// MX_PANEL columns: a panel's columns stay in registers, one per warp (lane l
+// holds rows l, l + 32, ...); each step updates them with one barrier, the owner
+// of the next column finding the next pivot and publishing its multiplier
+// column (look-ahead).  Then every other column is read once into registers, up
+// to six per warp, put through the panel's steps and written back.  Rows stay in
+// place (gj_pivot_publish); the output reads them back in pivot order.
+// At Ndim 112 an inverse takes 374 k cycles, half of it the 112 pivot steps'
+// latency; a step-by-step form (every column through shared memory each step,
+// 4-way selects instead of a branch on the pivot's row slot) took 597 k.  Same
+// operations per entry, in the same order.
+template <int R>
 __device__ __noinline__ int gj32_start(const double2* __restrict__ X, double2 w, int N,
                                        double2* __restrict__ const W, int iM, int iG,
                                        const MxShared s) {
+  constexpr int C = R == 2 ? 3 : 6;       // 16 warps x C columns >= 32 R - MX_PANEL
   const size_t NN = (size_t)N * N;
   double2* __restrict__ const Mi = W + iM * NN;
   double2* __restrict__ const G = W + iG * NN;
   SplitTail& sh = s.t();
-  const int T = blockDim.x, tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31, nwarp = T >> 5;
-  // pointers re-derived from the dynamic shared-memory array, so that the
-  // compiler emits shared-memory (not generic) loads and stores
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int nwarp = SP_T / 32;
   float2* __restrict__ sM = reinterpret_cast<float2*>(s.base());
-  float2* const cb0 = sh.colbuf;   // multiplier columns of even / odd steps
-  float2* const cb1 = sh.rowbuf;
+  float2* __restrict__ Cm = sM + (size_t)N * N;          // [MX_PANEL][N] multiplier columns
   float2* __restrict__ recip = sh.recip;
-  int* __restrict__ perm = sh.perm;
-  int* __restrict__ cols = sh.cols;
+  int* __restrict__ prow = sh.prow;                      // pivot rows of the panel's steps
   int* __restrict__ misc = sh.misc;
   int* __restrict__ pos_of = sh.pos_of;
   int* __restrict__ row_at = sh.row_at;
-  int rmax[4] = {0, 0, 0, 0};
+  int rmax[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) rmax[q] = 0;
+#pragma unroll 2
   for (int j = warp; j < N; j += nwarp) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < R; ++q) {
       const int i = lane + 32 * q;
       if (i < N) {
         const size_t e = (size_t)i + (size_t)j * N;
@@ -1132,7 +1194,7 @@ __device__ __noinline__ int gj32_start(const double2* __restrict__ X, double2 w,
   int* const eM = s.rows(iM, N);
   int* const eGr = s.rows(iG, N);
   int* const eGc = s.cols(iG, N);
-  for (int i = tid; i < N; i += T) {
+  for (int i = tid; i < N; i += SP_T) {
     pos_of[i] = i;
     row_at[i] = i;
     eM[i] = EXP_MIN;
@@ -1141,81 +1203,78 @@ __device__ __noinline__ int gj32_start(const double2* __restrict__ X, double2 w,
   if (tid == 0) misc[1] = 0;
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < R; ++q)
     if (lane + 32 * q < N) atomicMax(&eM[lane + 32 * q], rmax[q]);
-  if (warp == 0) {                        // step 0's pivot
-    float2 x[4];
+  for (int k0 = 0; k0 < N; k0 += MX_PANEL) {
+    const int pb = min(MX_PANEL, N - k0);
+    unsigned long long xp[1][R];          // this warp's panel column
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < R; ++m) {
       const int i = lane + 32 * m;
-      x[m] = i < N ? sM[i] : make_float2(0.f, 0.f);
+      const float2 v = (warp < pb && i < N) ? sM[(size_t)(k0 + warp) * N + i] : make_float2(0.f, 0.f);
+      xp[0][m] = pack2(v.x, v.y);
     }
-    gj_pivot_publish_u(x, 0, N, cb0, recip, perm, misc, pos_of, row_at);
-  }
-  __syncthreads();
-  for (int k = 0; k < N; ++k) {
+    auto publish = [&](int t) {
+      gj_pivot_publish<R>(xp[0], k0 + t, N, Cm + t * N, &recip[t], prow, misc, pos_of, row_at);
+    };
+    if (warp == 0) publish(0);
+    __syncthreads();
+    for (int t = 0; t < pb; ++t) {
+      if (misc[1]) break;
+      if (warp < pb) {
+        gj_step_cols<R, 1>(xp, Cm + t * N, N, prow[k0 + t], recip[t], warp == t ? 0 : -1);
+        if (warp == t + 1) publish(t + 1);
+      }
+      __syncthreads();
+    }
     if (misc[1]) break;
-    const int p = misc[2 + (k & 1)];        // the pivot's row
-    const float2 r = recip[k & 1];
-    const float2* cb = (k & 1) ? cb1 : cb0;
-    float2* cbn = (k & 1) ? cb0 : cb1;
-    float2 f[4];                          // this lane's multipliers
+    if (warp < pb) {                      // panel column back to shared memory
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int i = lane + 32 * m;
-      f[m] = i < N ? cb[i] : make_float2(0.f, 0.f);
+      for (int m = 0; m < R; ++m) {
+        const int i = lane + 32 * m;
+        if (i < N) sM[(size_t)(k0 + warp) * N + i] = unpack2(xp[0][m]);
+      }
     }
-    for (int j = warp; j < N; j += nwarp) {
-      float2* col = sM + (size_t)j * N;
-      float2 x[4];
+    // this warp's other columns through the panel's steps
+    const int nt = N - pb, nc = warp < nt ? (nt - warp + nwarp - 1) / nwarp : 0;
+    if (nc > 0) {
+      unsigned long long x[C][R];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const int i = lane + 32 * m;
-        x[m] = i < N ? col[i] : make_float2(0.f, 0.f);
-      }
-      float2 nk = r;
-      if (j == k) {                       // the pivot column becomes a column of the inverse
+      for (int c = 0; c < C; ++c) {
+        const int o = warp + c * nwarp;
+        const float2* col = sM + (size_t)(o < k0 ? o : o + pb) * N;
 #pragma unroll
-        for (int m = 0; m < 4; ++m) x[m] = make_float2(0.f, 0.f);
-      } else {
-        const float2 apj = shfl_f2c(pick4(x, p >> 5), p & 31);
-        nk = make_float2(fmaf(apj.x, r.x, -apj.y * r.y), fmaf(apj.x, r.y, apj.y * r.x));
+        for (int m = 0; m < R; ++m) {
+          const int i = lane + 32 * m;
+          const float2 v = (c < nc && i < N) ? col[i] : make_float2(0.f, 0.f);
+          x[c][m] = pack2(v.x, v.y);
+        }
       }
+      for (int t = 0; t < pb; ++t)
+        gj_step_cols<R, C>(x, Cm + t * N, N, prow[k0 + t], recip[t], -1);
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const int i = lane + 32 * m;
-        float2 v = x[m];
-        v.x = fmaf(-f[m].x, nk.x, v.x);
-        v.x = fmaf(f[m].y, nk.y, v.x);
-        v.y = fmaf(-f[m].x, nk.y, v.y);
-        v.y = fmaf(-f[m].y, nk.x, v.y);
-        x[m] = (i == p) ? nk : v;
-        if (i < N) col[i] = x[m];
+      for (int c = 0; c < C; ++c) {
+        const int o = warp + c * nwarp;
+        float2* col = sM + (size_t)(o < k0 ? o : o + pb) * N;
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+          const int i = lane + 32 * m;
+          if (c < nc && i < N) col[i] = unpack2(x[c][m]);
+        }
       }
-      if (j == k + 1) gj_pivot_publish_u(x, k + 1, N, cbn, recip, perm, misc, pos_of, row_at);
     }
     __syncthreads();
   }
   const int singular = misc[1];
-  if (tid == 0) {
-    for (int j = 0; j < N; ++j) cols[j] = j;
-    if (!singular) {
-      for (int k = N - 1; k >= 0; --k) {
-        const int p = perm[k];
-        const int t = cols[k];
-        cols[k] = cols[p];
-        cols[p] = t;
-      }
-    }
-  }
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < 4; ++q) rmax[q] = 0;
+  for (int q = 0; q < R; ++q) rmax[q] = 0;
+#pragma unroll 2
   for (int j = warp; j < N; j += nwarp) {
-    const int cj = cols[j];
+    const int cj = pos_of[j];             // the row swaps as column swaps of the inverse
     int cmax = EXP_MIN;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < R; ++q) {
       const int i = lane + 32 * q;
       if (i < N) {
         double2 g = make_double2(i == j ? 1.0 : 0.0, 0.0);
@@ -1233,104 +1292,10 @@ __device__ __noinline__ int gj32_start(const double2* __restrict__ X, double2 w,
     if (lane == 0) eGc[j] = cmax;
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < R; ++q)
     if (lane + 32 * q < N) atomicMax(&eGr[lane + 32 * q], rmax[q]);
   __syncthreads();
   return singular;
-}
-
-template <int R>
-__device__ __forceinline__ float2 pick_f(const float2 (&x)[R], int m) {
-  float2 v = x[0];
-#pragma unroll
-  for (int q = 1; q < R; ++q)
-    if (q == m) v = x[q];
-  return v;
-}
-
-__device__ __forceinline__ float2 shfl_f2(float2 v, int src) {
-  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-
-// gj_pivot_publish_u for a column of R rows per lane (rows lane + 32 m): the
-// multiplier column goes to cb, the reciprocal to *rslot, the pivot's row to
-// prow[t]
-template <int R>
-__device__ __forceinline__ void gj_pivot_publish_ur(const float2 (&x)[R], int t, int N, float2* cb,
-                                                 float2* rslot, int* perm, int* prow, int* misc,
-                                                 int* pos_of, int* row_at) {
-  const int lane = threadIdx.x & 31;
-  int bkey = -1, bpos = 0x7fffffff, brow = N;
-#pragma unroll
-  for (int m = 0; m < R; ++m) {
-    const int i = lane + 32 * m;
-    if (i < N) {
-      const int ps = pos_of[i];
-      const int key = __float_as_int(fabsf(x[m].x) + fabsf(x[m].y));
-      if (ps >= t && (key > bkey || (key == bkey && ps < bpos))) {
-        bkey = key;
-        bpos = ps;
-        brow = i;
-      }
-    }
-  }
-  {  // warp maximum of the key, then the smallest position among the lanes that hold it
-    const unsigned kmax = __reduce_max_sync(0xffffffffu, (unsigned)(bkey + 1));
-    const bool cand = (unsigned)(bkey + 1) == kmax;
-    const int pmin = (int)__reduce_min_sync(0xffffffffu, cand ? (unsigned)bpos : 0xffffffffu);
-    const int src = __ffs(__ballot_sync(0xffffffffu, cand && bpos == pmin)) - 1;
-    brow = __shfl_sync(0xffffffffu, brow, src);
-    bkey = (int)kmax - 1;
-    bpos = pmin;
-  }
-  const float2 xp = shfl_f2(pick_f<R>(x, brow >> 5), brow & 31);
-#pragma unroll
-  for (int m = 0; m < R; ++m) {
-    const int i = lane + 32 * m;
-    if (i < N) cb[i] = x[m];
-  }
-  if (lane == 0) {
-    perm[t] = bpos;
-    prow[t] = brow;
-    const int rk = row_at[t];
-    row_at[bpos] = rk;
-    pos_of[rk] = bpos;
-    row_at[t] = brow;
-    pos_of[brow] = t;
-    if (bkey == 0) {
-      misc[1] = 1;
-    } else {
-      const float inv_d = 1.0f / (xp.x * xp.x + xp.y * xp.y);
-      *rslot = make_float2(xp.x * inv_d, -xp.y * inv_d);
-    }
-  }
-}
-
-// one Gauss-Jordan step k (pivot row p, reciprocal r, multiplier column cm in
-// shared memory) applied to column j held in registers, rows in place
-template <int R>
-__device__ __forceinline__ void gj_step_col_u(float2 (&x)[R], const float2* __restrict__ cm, int N,
-                                              int j, int k, int p, float2 r) {
-  const int lane = threadIdx.x & 31;
-  float2 nk = r;
-  if (j == k) {
-#pragma unroll
-    for (int m = 0; m < R; ++m) x[m] = make_float2(0.f, 0.f);
-  } else {
-    const float2 apj = shfl_f2(pick_f<R>(x, p >> 5), p & 31);
-    nk = make_float2(fmaf(apj.x, r.x, -apj.y * r.y), fmaf(apj.x, r.y, apj.y * r.x));
-  }
-#pragma unroll
-  for (int m = 0; m < R; ++m) {
-    const int i = lane + 32 * m;
-    const float2 f = i < N ? cm[i] : make_float2(0.f, 0.f);
-    float2 v = x[m];
-    v.x = fmaf(-f.x, nk.x, v.x);
-    v.x = fmaf(f.y, nk.y, v.x);
-    v.y = fmaf(-f.x, nk.y, v.y);
-    v.y = fmaf(-f.y, nk.x, v.y);
-    x[m] = (i == p) ? nk : v;
-  }
 }
 
 // As gj32_start for Ndim above the shared-memory limit: the FP32 matrix lives
@@ -1349,16 +1314,15 @@ __device__ __noinline__ int gj32_global(const double2* __restrict__ X, double2 w
   double2* __restrict__ const Mi = W + iM * NN;
   double2* __restrict__ const G = W + iG * NN;
   SplitTail& sh = s.t();
-  const int T = blockDim.x, tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31, nwarp = T >> 5;
+  constexpr int C = R <= 5 ? 3 : 2;       // columns a warp takes at a time
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int nwarp = SP_T / 32;
   float2* __restrict__ const Wf = reinterpret_cast<float2*>(W + iW * NN);
   // [MX_MAXN][MX_PANEL] multiplier columns of the panel
   float2* __restrict__ Cm = reinterpret_cast<float2*>(s.base());
   float2* __restrict__ recip = sh.recip;
-  int* __restrict__ perm = sh.perm;
-  int* __restrict__ cols = sh.cols;
   int* __restrict__ misc = sh.misc;
-  int* const prow = cols;                        // pivot rows during the steps
+  int* const prow = sh.prow;                     // pivot rows of the steps
   int* __restrict__ pos_of = sh.pos_of;
   int* __restrict__ row_at = sh.row_at;
   int rmax[R];
@@ -1382,7 +1346,7 @@ __device__ __noinline__ int gj32_global(const double2* __restrict__ X, double2 w
   int* const eM = s.rows(iM, N);
   int* const eGr = s.rows(iG, N);
   int* const eGc = s.cols(iG, N);
-  for (int i = tid; i < N; i += T) {
+  for (int i = tid; i < N; i += SP_T) {
     pos_of[i] = i;
     row_at[i] = i;
     eM[i] = EXP_MIN;
@@ -1395,82 +1359,73 @@ __device__ __noinline__ int gj32_global(const double2* __restrict__ X, double2 w
     if (lane + 32 * q < N) atomicMax(&eM[lane + 32 * q], rmax[q]);
   for (int k0 = 0; k0 < N; k0 += MX_PANEL) {
     const int pb = min(MX_PANEL, N - k0);
-    float2 xc[2][R];                // this warp's panel columns warp, warp + nwarp
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-      const int c = warp + cc * nwarp;
+    {
+      unsigned long long xp[1][R];        // this warp's panel column
+      float2* const col = Wf + (size_t)(k0 + warp) * N;
 #pragma unroll
       for (int m = 0; m < R; ++m) {
         const int i = lane + 32 * m;
-        xc[cc][m] = (c < pb && i < N) ? Wf[(size_t)(k0 + c) * N + i] : make_float2(0.f, 0.f);
+        const float2 v = (warp < pb && i < N) ? col[i] : make_float2(0.f, 0.f);
+        xp[0][m] = pack2(v.x, v.y);
       }
-    }
-    if (warp == 0) gj_pivot_publish_ur<R>(xc[0], k0, N, Cm, &recip[0], perm, prow, misc, pos_of, row_at);
-    __syncthreads();
-    for (int t = 0; t < pb; ++t) {
-      if (misc[1]) break;
-      const int k = k0 + t, p = prow[k];
-      const float2 r = recip[t];
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c = warp + cc * nwarp;
-        if (c < pb) {
-          gj_step_col_u<R>(xc[cc], Cm + t * N, N, k0 + c, k, p, r);
-          if (c == t + 1)
-            gj_pivot_publish_ur<R>(xc[cc], k + 1, N, Cm + (t + 1) * N, &recip[t + 1], perm, prow, misc,
-                                   pos_of, row_at);
-        }
-      }
+      auto publish = [&](int t) {
+        gj_pivot_publish<R>(xp[0], k0 + t, N, Cm + t * N, &recip[t], prow, misc, pos_of, row_at);
+      };
+      if (warp == 0) publish(0);
       __syncthreads();
-    }
-    if (misc[1]) break;
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {       // panel columns back to memory
-      const int c = warp + cc * nwarp;
-      if (c < pb) {
+      for (int t = 0; t < pb; ++t) {
+        if (misc[1]) break;
+        if (warp < pb) {
+          gj_step_cols<R, 1>(xp, Cm + t * N, N, prow[k0 + t], recip[t], warp == t ? 0 : -1);
+          if (warp == t + 1) publish(t + 1);
+        }
+        __syncthreads();
+      }
+      if (misc[1]) break;
+      if (warp < pb) {                    // panel column back to memory
 #pragma unroll
         for (int m = 0; m < R; ++m) {
           const int i = lane + 32 * m;
-          if (i < N) Wf[(size_t)(k0 + c) * N + i] = xc[cc][m];
+          if (i < N) col[i] = unpack2(xp[0][m]);
         }
       }
     }
-    // every column outside the panel through the panel's steps, in registers
-    for (int j = warp; j < N; j += nwarp) {
-      if (j >= k0 && j < k0 + pb) continue;
-      float2* col = Wf + (size_t)j * N;
-      float2 x[R];
+    // every column outside the panel through the panel's steps, C at a time
+    for (int o0 = warp; o0 < N - pb; o0 += C * nwarp) {
+      const int nc = min(C, (N - pb - o0 + nwarp - 1) / nwarp);
+      unsigned long long x[C][R];
 #pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const int i = lane + 32 * q;
-        x[q] = i < N ? col[i] : make_float2(0.f, 0.f);
+      for (int c = 0; c < C; ++c) {
+        const int o = o0 + c * nwarp;
+        const float2* col = Wf + (size_t)(o < k0 ? o : o + pb) * N;
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+          const int i = lane + 32 * m;
+          const float2 v = (c < nc && i < N) ? col[i] : make_float2(0.f, 0.f);
+          x[c][m] = pack2(v.x, v.y);
+        }
       }
-      for (int t = 0; t < pb; ++t) gj_step_col_u<R>(x, Cm + t * N, N, j, k0 + t, prow[k0 + t], recip[t]);
+      for (int t = 0; t < pb; ++t)
+        gj_step_cols<R, C>(x, Cm + t * N, N, prow[k0 + t], recip[t], -1);
 #pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const int i = lane + 32 * q;
-        if (i < N) col[i] = x[q];
+      for (int c = 0; c < C; ++c) {
+        const int o = o0 + c * nwarp;
+        float2* col = Wf + (size_t)(o < k0 ? o : o + pb) * N;
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+          const int i = lane + 32 * m;
+          if (c < nc && i < N) col[i] = unpack2(x[c][m]);
+        }
       }
     }
     __syncthreads();
   }
   const int singular = misc[1];
-  if (tid == 0) {
-    for (int j = 0; j < N; ++j) cols[j] = j;
-    if (!singular) {
-      for (int k = N - 1; k >= 0; --k) {
-        const int p = perm[k];
-        const int t = cols[k];
-        cols[k] = cols[p];
-        cols[p] = t;
-      }
-    }
-  }
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < R; ++q) rmax[q] = 0;
   for (int j = warp; j < N; j += nwarp) {
-    const int cj = cols[j];
+    const int cj = pos_of[j];             // the row swaps as column swaps of the inverse
     int cmax = EXP_MIN;
 #pragma unroll
     for (int q = 0; q < R; ++q) {
@@ -1500,7 +1455,8 @@ __device__ __noinline__ int gj32_global(const double2* __restrict__ X, double2 w
 // FP32 inverse of w I - X by Ndim: M to workspace matrix iM, the inverse to iG, iR as work
 __device__ __forceinline__ int gj32(const double2* X, double2 w, int N, double2* W, int iM, int iG,
                                     int iR, const MxShared s) {
-  return N <= MX_SMEM_GJ_N ? gj32_start(X, w, N, W, iM, iG, s)
+  return N <= 64              ? gj32_start<2>(X, w, N, W, iM, iG, s)
+         : N <= MX_SMEM_GJ_N ? gj32_start<4>(X, w, N, W, iM, iG, s)
          : N <= 160        ? gj32_global<5>(X, w, N, W, iM, iG, iR, s)
          : N <= 224        ? gj32_global<7>(X, w, N, W, iM, iG, iR, s)
                            : gj32_global<MX_ROWS>(X, w, N, W, iM, iG, iR, s);
