@@ -42,12 +42,12 @@ __host__ __device__ inline MxPlan mx_plan(int N, int w0_req = 0) {
 
 __device__ __forceinline__ float gemm7(double2* W, uint32_t op, int epi, int epi2, const MxPlan& p,
                                        const MxShared s) {
-  return split_gemm<Dig7>(W, op, epi, epi2, p.N, p.NP, p.w0, p.ncb, s);
+  return split_gemm<Dig7>(W, op, epi, epi2, p.N, p.NP, p.w0, s);
 }
 __device__ __forceinline__ void gemm4(double2* W, uint32_t op, int epi, const MxPlan& p7,
                                       const MxShared s) {
   const MxPlan p = split_plan4(p7);
-  split_gemm<Dig4>(W, op, epi, -1, p.N, p.NP, p.w0, p.ncb, s);
+  split_gemm<Dig4>(W, op, epi, -1, p.N, p.NP, p.w0, s);
 }
 
 // (w I - X)^-1 into workspace matrix G: FP32 Gauss-Jordan, then Newton-Schulz
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(MX_T, 1) k_mixed_unit(int op, int N, double2* 
     for (int e = tid; e < NN; e += blockDim.x) negX[e] = make_double2(-W[e].x, -W[e].y);
     __syncthreads();
     int G = 3, Gn = 4;
-    sing = mixed_inverse(negX, make_double2(0.0, 0.0), W, pl, ns, G, Gn, 5, 6, s);
+    sing = mixed_inverse(negX, make_double2(0.0, 0.0), W, pl, ns, G, Gn, 6, 5, s);
     double2* C = W + 2 * (size_t)NN;
     for (int e = tid; e < NN; e += blockDim.x) C[e] = W[(size_t)G * NN + e];
   }

@@ -31,8 +31,9 @@
 // tensor pipe at 60-80 %.
 //
 // Digits are made from packed integer extraction and one packed 16-bit
-// floating-point instruction per two digits (a digit's bits under a fixed
-// exponent, minus the offset: exact), 4-6 instructions per pair of digits.
+// floating-point FMA per two digits (a digit's bits under a fixed exponent,
+// minus the offset: exact).  Generation and drain are bound by the integer pipe
+// (64 lanes a clock per SM), so both are written for few integer instructions.
 //
 // Every mbarrier wait is bounded; on a timeout the CTA stops issuing work,
 // marks the instance, waits (bounded) for its MMAs and frees tensor memory.
@@ -169,6 +170,25 @@ __device__ __forceinline__ double assemble(long long S, int be0) {
   return __longlong_as_double((long long)(r | ((unsigned long long)sg << 63)));
 }
 
+// assemble for |S| < 2^63, with the common case (zero, or |S| >= 2^32 and a normal
+// result) in about half the instructions: the drain of the accumulators is
+// bound by the integer pipe
+template <bool ROUND>
+__device__ __forceinline__ double assemble_fast(long long S, int be0) {
+  const long long sg = S >> 63;
+  const unsigned long long a = (unsigned long long)((S ^ sg) - sg);
+  const unsigned ah = (unsigned)(a >> 32);
+  const int lz = __clz((int)ah);
+  const int be = 63 - lz + be0;
+  if (a != 0 && (ah == 0 || (unsigned)(be - 1) >= 2045u)) return assemble<ROUND>(S, be0);
+  unsigned long long n = a << ((lz - 1) & 63);        // leading bit at 62
+  if (ROUND) n += 0x200;
+  const unsigned long long m = n >> 10;               // the hidden bit adds 1 to the exponent
+  const unsigned hi = ((unsigned)(m >> 32) + ((unsigned)(be - 1) << 20)) |
+                      ((unsigned)(sg >> 32) & 0x80000000u);
+  return __hiloint2double((int)(a != 0 ? hi : 0u), (int)(a != 0 ? (unsigned)m : 0u));
+}
+
 __device__ __forceinline__ float d2f_bits(double x) {    // truncating FP64 -> FP32
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const uint32_t sign = (uint32_t)(u >> 63) << 31;
@@ -193,9 +213,9 @@ __device__ __forceinline__ double f2d_bits(float f) {     // exact FP32 -> FP64
 // ---- digit kinds -------------------------------------------------------------
 
 // packed 16-bit floating point on raw words
-__device__ __forceinline__ uint32_t hadd2_f16(uint32_t a, uint32_t b) {
+__device__ __forceinline__ uint32_t hfma2_f16(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t r;
-  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
   return r;
 }
 __device__ __forceinline__ uint32_t hfma2_bf16(uint32_t a, uint32_t b, uint32_t c) {
@@ -275,6 +295,12 @@ struct DigB7 {
   static __device__ __forceinline__ void digits_b(double x0, double x1, int E, uint32_t (&w)[D]) {
     digits<5>(x0, x1, E, w);
   }
+  static __device__ __forceinline__ void digits_pm(double x0, double x1, int E, uint32_t (&w)[D],
+                                                   uint32_t (&wn)[D]) {
+    digits<5>(x0, x1, E, w);
+#pragma unroll
+    for (int p = 0; p < D; ++p) wn[p] = w[p] ^ 0x80008000u;
+  }
   template <int T>
   static __device__ __forceinline__ int m_of(uint32_t v) {
     return __float2int_rz(__uint_as_float(v) * __int_as_float((127 + 7 * T - 56) << 23));
@@ -291,15 +317,15 @@ struct DigB7 {
       S += a == 0 ? (long long)((unsigned long long)(long long)m << 35)
                   : (long long)m * (1ll << (49 - 7 * (a + 2)));
     }
-    return assemble<false>(S, ee - 1070);
+    return assemble_fast<false>(S, ee - 1070);
   }
 };
 
-// Base-256 digits as F16.  x = F 2^(E - 1022 - 54), |F| <= 2^54 rounded to
-// nearest (ties away from zero); F + 128 (1 + 256 + .. + 256^6) has byte digits
-// g_p, and F = sum of (g_p - 128) 256^(7-p): the leading digit is in [-64, 64],
-// the others in [-128, 127].  An F16 word 0x6400 | g is 1024 + g, so 1024 + g -
-// 1152 is the digit, exactly, by one packed add.  Order t gathers 2 (t - 1) K
+// Base-256 digits as F16.  |x| = F 2^(E - 1022 - 54), F <= 2^54 rounded to
+// nearest; F + 128 (1 + 256 + .. + 256^6) has byte digits g_p, and F = sum of
+// (g_p - 128) 256^(7-p): the leading digit is in [0, 64], the others in
+// [-128, 127].  An F16 word 0x6400 | g is 1024 + g, so (1024 + g) s - 1152 s is
+// the digit times the element's sign s, exactly, by one packed FMA.  Order t gathers 2 (t - 1) K
 // digit products of at most 2^12 (1, 1), 2^13 (1, q) or 2^14: below 2^24 for
 // the orders 2..5 at K <= 170 and order 6 at K <= 128 even with every product
 // at its bound and of one sign; above that, K is accumulated in parts of at
@@ -323,59 +349,84 @@ struct DigF8 {
   struct Fix {
     uint32_t lo, hi;                                  // bytes g_7 .. g_4 | g_3 g_2 g_1 0x64
   };
+  // |x|: (((|x| 2^(55 - E + 1022)) truncated) + 1) / 2 = |F|
   static __device__ __forceinline__ Fix fix(double x, int E) {
     const unsigned long long u = (unsigned long long)__double_as_longlong(x);
     const int ex = (int)(u >> 52) & 0x7FF;
-    const unsigned long long t = shr64(signif(u) << 2, (unsigned)(E - ex));
-    const unsigned long long s = (unsigned long long)((long long)u >> 63);
-    // x >= 0: (t + 1) >> 1 = F; x < 0: (-t) >> 1 = -F
-    const unsigned long long v = ((t ^ s) + (1 + 2 * BIAS + (0x64ull << 57))) >> 1;
+    const unsigned long long v =
+        (shr64(signif(u) << 2, (unsigned)(E - ex)) + (1 + 2 * BIAS + (0x64ull << 57))) >> 1;
     return Fix{(uint32_t)v, (uint32_t)(v >> 32)};
   }
   template <int P>
-  static __device__ __forceinline__ uint32_t digit(const Fix& a, const Fix& b) {
-    uint32_t g;
+  static __device__ __forceinline__ uint32_t biased(const Fix& a, const Fix& b) {
     if constexpr (P <= 3) {
       constexpr uint32_t j = 3 - P;
-      g = __byte_perm(a.hi, b.hi, j | 0x30u | ((4 + j) << 8) | 0x7000u);
+      return __byte_perm(a.hi, b.hi, j | 0x30u | ((4 + j) << 8) | 0x7000u);
     } else {
       constexpr uint32_t j = 7 - P;
-      g = (__byte_perm(a.lo, b.lo, j | (j << 4) | ((4 + j) << 8) | ((4 + j) << 12)) &
-           0x00FF00FFu) | 0x64006400u;
+      return (__byte_perm(a.lo, b.lo, j | (j << 4) | ((4 + j) << 8) | ((4 + j) << 12)) &
+              0x00FF00FFu) | 0x64006400u;
     }
-    return hadd2_f16(g, 0xE480E480u);                 // - 1152
+  }
+  // the D digit words of a pair of reals and, with NEG, their negatives
+  template <bool NEG>
+  static __device__ __forceinline__ void digits(double x0, double x1, int E, uint32_t (&w)[D],
+                                                uint32_t (&wn)[D]) {
+    const Fix a = fix(x0, E), b = fix(x1, E);
+    uint32_t g[D];
+    g[0] = biased<1>(a, b);
+    g[1] = biased<2>(a, b);
+    g[2] = biased<3>(a, b);
+    g[3] = biased<4>(a, b);
+    if constexpr (D > 4) {
+      g[4] = biased<5>(a, b);
+      g[5] = biased<6>(a, b);
+      g[6] = biased<7>(a, b);
+    }
+    // +-1 and -+1152 by the elements' signs, as F16 pairs
+    const uint32_t sg = __byte_perm((uint32_t)__double2hiint(x0), (uint32_t)__double2hiint(x1), 0x7632) &
+                        0x80008000u;
+    const uint32_t one = sg | 0x3C003C00u, off = sg ^ 0xE480E480u;
+#pragma unroll
+    for (int p = 0; p < D; ++p) {
+      w[p] = hfma2_f16(g[p], one, off);
+      if (NEG) wn[p] = hfma2_f16(g[p], one ^ 0x80008000u, off ^ 0x80008000u);
+    }
   }
   static __device__ __forceinline__ void digits_a(double x0, double x1, int E, uint32_t (&w)[D]) {
-    const Fix a = fix(x0, E), b = fix(x1, E);
-    w[0] = digit<1>(a, b);
-    w[1] = digit<2>(a, b);
-    w[2] = digit<3>(a, b);
-    w[3] = digit<4>(a, b);
-    if constexpr (D > 4) {
-      w[4] = digit<5>(a, b);
-      w[5] = digit<6>(a, b);
-      w[6] = digit<7>(a, b);
-    }
+    digits<false>(x0, x1, E, w, w);
   }
   static __device__ __forceinline__ void digits_b(double x0, double x1, int E, uint32_t (&w)[D]) {
-    digits_a(x0, x1, E, w);
+    digits<false>(x0, x1, E, w, w);
+  }
+  static __device__ __forceinline__ void digits_pm(double x0, double x1, int E, uint32_t (&w)[D],
+                                                   uint32_t (&wn)[D]) {
+    digits<true>(x0, x1, E, w, wn);
   }
   static __device__ __forceinline__ int f2i(uint32_t v) {
     return __float2int_rz(__uint_as_float(v));
   }
-  static __device__ __forceinline__ long long part(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    return (long long)f2i(a) * (1ll << 24) + ((long long)f2i(b) * (1ll << 16) +
-           ((long long)f2i(c) * (1ll << 8) + (long long)f2i(d)));
-  }
+  // value of the accumulators of one output component
   static __device__ __forceinline__ double value(const uint32_t (&v)[NACC], int ee) {
     // order t in units of 256^(14-t) 2^(ee - 2152)
-    const long long hi = part(v[0], v[1], v[2], v[3]);
     if constexpr (D > 4) {
-      const long long lo = part(v[4], v[5], v[6], v[7]);
-      // hi 2^32 + lo, rounded to units of 2^14: |hi| < 2^45
-      return assemble<true>((hi << 18) + ((lo + (1ll << 13)) >> 14), ee - 2152 + 54 + 1023);
+      // the sum in units of 256^5 2^14, a quarter of order 7's: |sum| < 2^63.  The orders
+      // 7..9 are added in FP32 (2^-24 of order 7, at most 2^-58 of the scales for
+      // partial sums of random digits) and converted together; order 2, below
+      // 2^22, is converted by an add (conversions run at 16 a clock per SM)
+      const float f789 = fmaf(__uint_as_float(v[7]), 0x1p-14f,
+                              fmaf(__uint_as_float(v[6]), 0x1p-6f, 4.0f * __uint_as_float(v[5])));
+      const int low = __float2int_rn(f789);
+      const int m2 = __float_as_int(__uint_as_float(v[0]) + 12582912.0f);      // + 0x4B400000
+      const long long S = ((long long)f2i(v[2]) * (1ll << 26) + (long long)f2i(v[3]) * (1ll << 18)) +
+                          ((long long)f2i(v[4]) * (1ll << 10) + (long long)low);
+      const unsigned top = (unsigned)m2 * 1024u + ((unsigned)f2i(v[1]) * 4u);  // in units of 2^32
+      return assemble_fast<true>(S + (long long)((unsigned long long)top << 32),
+                                 ee - 2152 + 54 + 1023);
     } else {
-      return assemble<true>(hi, ee - 2152 + 72 + 1023);
+      const long long S = ((long long)f2i(v[0]) * (1ll << 24) + (long long)f2i(v[1]) * (1ll << 16)) +
+                          ((long long)f2i(v[2]) * (1ll << 8) + (long long)f2i(v[3]));
+      return assemble_fast<true>(S, ee - 2152 + 72 + 1023);
     }
   }
 };
@@ -642,40 +693,56 @@ __host__ __device__ constexpr uint32_t ops(int X, int Y, int out, int aux = 0, i
 __device__ __forceinline__ int item_row(int it) { return (it >> 6) * 8 + ((it & 31) >> 2); }
 __device__ __forceinline__ int item_k(int it) { return ((it >> 5) & 1) * 8 + (it & 3) * 2; }
 
-// The tiles of one product and their chunks.  A tile is a row block of 128, a
-// column pass and a part of K (K part fastest, then the pass, then the row
-// block); its chunks are 16 of K.
-struct Tiles {
-  int N, NP, w0, ncb, M, nks, kper;
-  __device__ __forceinline__ int count() const { return ((M + 127) / 128) * ncb * nks; }
-  __device__ __forceinline__ int chunks(int ks) const {
-    return (min(N, (ks + 1) * kper) - ks * kper + KCH - 1) / KCH;
-  }
+// A tile of a product: a row block of 128, a column pass and a part of K; its
+// chunks are 16 of K.  next() steps through a product's tiles (K part fastest,
+// then the pass, then the row block) without divisions: a product at Ndim 40 has
+// two tiles of three chunks, and the position arithmetic was a tenth of it.
+struct Tile {
+  int rb0, jb, width, ka, kb;
+  __device__ __forceinline__ int chunks() const { return (kb - ka + KCH - 1) / KCH; }
 };
 template <class K>
-__device__ __forceinline__ Tiles tiles_of(int N, int NP, int w0, int ncb, bool stack) {
+__device__ __forceinline__ int k_part(int N) {       // K of one part
   const int nks = (N + K::KSPLIT - 1) / K::KSPLIT;
-  const int kper = nks == 1 ? N : (((N + nks - 1) / nks + KCH - 1) & ~(KCH - 1));
-  return Tiles{N, NP, w0, ncb, stack ? 2 * N : N, nks, kper};
+  return nks <= 1 ? N : (((N + nks - 1) / nks + KCH - 1) & ~(KCH - 1));
+}
+__device__ __forceinline__ Tile first_tile(int N, int NP, int w0, int kper) {
+  return Tile{0, 0, min(w0, NP), 0, min(N, kper)};
+}
+// false: t was the last tile (it is left as it is)
+__device__ __forceinline__ bool next_tile(Tile& t, int M, int N, int NP, int w0, int kper) {
+  if (t.kb < N) {
+    t.ka = t.kb;
+    t.kb = min(N, t.kb + kper);
+    return true;
+  }
+  if (t.jb + w0 < NP) {
+    t.jb += w0;
+  } else {
+    if (t.rb0 + 128 >= M) return false;
+    t.rb0 += 128;
+    t.jb = 0;
+  }
+  t.width = min(w0, NP - t.jb);
+  t.ka = 0;
+  t.kb = min(N, kper);
+  return true;
 }
 
-// Digit planes of tile t's chunks gc .. ge-1 (warps 1..15), chunk gc being
+// Digit planes of a tile's chunks gc .. ge-1 (warps 1..15), chunk gc being
 // number `chunk` of the kernel's chunk sequence.  Returns 1 when a wait gave up.
 // A function of its own (as split_drain), so that neither phase's registers are
 // live in the other: one function for both spilled.
 template <class K>
 __device__ __noinline__ int split_generate(const double2* __restrict__ W, uint32_t op, int N,
-                                           int NP, int w0, int ncb, int stack, int t, int gc,
-                                           int ge, uint32_t chunk, MxShared s) {
+                                           int M, Tile T, int gc, int ge, uint32_t chunk,
+                                           MxShared s) {
   constexpr int D = K::D;
   constexpr int NR = D == 7 ? 3 : 4;             // rounds of items per generating thread
   SplitTail& sh = s.t();
-  const Tiles T = tiles_of<K>(N, NP, w0, ncb, stack);
-  const size_t NN = (size_t)N * N;
+  const int NN = N * N;
   const int gtid = threadIdx.x - 32, lane = threadIdx.x & 31;
-  const int ks = t % T.nks, u = t / T.nks, cb = u % ncb;
-  const int rb0 = (u / ncb) * 128, jb = cb * w0, width = min(w0, NP - jb);
-  const int ka = ks * T.kper, kb = min(N, ka + T.kper);
+  const int width = T.width, ka = T.ka, kb = T.kb;
   // this thread's items: element address at chunk gc, distance of the pair's
   // second element, shared exponent (address null: zeros)
   const double2* px[NR];
@@ -687,17 +754,17 @@ __device__ __noinline__ int split_generate(const double2* __restrict__ W, uint32
     ex[r] = EXP_MIN;
     const int k = ka + gc * KCH + item_k(it);    // 1024 is a multiple of 64: the same for B items
     if (it < 1024) {
-      const int i = rb0 + item_row(it);
-      if (i < T.M) {
-        const bool low = stack && i >= N;
+      const int i = T.rb0 + item_row(it);
+      if (i < M) {
+        const bool low = i >= N;                 // the second product's rows of a stacked pair
         const int m = low ? (op >> 16) & 15 : op & 15, il = low ? i - N : i;
-        px[r] = W + m * NN + il + (size_t)k * N;
+        px[r] = W + (size_t)(m * NN) + il + k * N;
         ex[r] = s.rows(m, N)[il];
       }
     } else if (it - 1024 < width * 8) {
-      const int j = jb + item_row(it - 1024), m = (op >> 4) & 15;
+      const int j = T.jb + item_row(it - 1024), m = (op >> 4) & 15;
       if (j < N) {
-        px[r] = W + m * NN + (size_t)j * N + k;
+        px[r] = W + (size_t)(m * NN) + j * N + k;
         ex[r] = s.cols(m, N)[j];
       }
     }
@@ -713,7 +780,7 @@ __device__ __noinline__ int split_generate(const double2* __restrict__ W, uint32
       if (px[r]) {
         if (k < kb) raw[r][0] = *px[r];
         if (k + 1 < kb) raw[r][1] = px[r][it < 1024 ? N : 1];
-        px[r] += it < 1024 ? (size_t)KCH * N : (size_t)KCH;
+        px[r] += it < 1024 ? KCH * N : KCH;
       }
     }
   };
@@ -729,6 +796,11 @@ __device__ __noinline__ int split_generate(const double2* __restrict__ W, uint32
       uint32_t w[D];
       if (it < 1024) {
         uint32_t* const dst = reinterpret_cast<uint32_t*>(A) + it;
+        if (__all_sync(0xffffffffu, px[r] == nullptr)) {     // 8 padding rows of the tile
+#pragma unroll
+          for (int p = 0; p < 2 * D; ++p) dst[p * (APLANE / 4)] = 0u;
+          continue;
+        }
         K::digits_a(raw[r][0].x, raw[r][1].x, ex[r], w);
 #pragma unroll
         for (int p = 0; p < D; ++p) dst[2 * p * (APLANE / 4)] = w[p];
@@ -747,13 +819,14 @@ __device__ __noinline__ int split_generate(const double2* __restrict__ W, uint32
           *d0 = w[p];
           *d1 = w[p];
         }
-        K::digits_b(raw[r][0].y, raw[r][1].y, ex[r], w);
+        uint32_t wn[D];
+        K::digits_pm(raw[r][0].y, raw[r][1].y, ex[r], w, wn);
         d0 = dst + bs;
         d1 = dst + 2 * D * bs;
 #pragma unroll
         for (int p = 0; p < D; ++p, d0 += 2 * bs, d1 += 2 * bs) {
           *d0 = w[p];
-          *d1 = w[p] ^ 0x80008000u;
+          *d1 = wn[p];
         }
       }
     }
@@ -765,27 +838,24 @@ __device__ __noinline__ int split_generate(const double2* __restrict__ W, uint32
   return 0;
 }
 
-// Accumulators of tile t through the epilogue (all warps: four per quadrant of
+// Accumulators of a tile through the epilogue (all warps: four per quadrant of
 // 32 tensor-memory lanes, each taking 4 of every 16 columns).  Returns this
 // thread's part of the product's FP32 sum.
 template <class K>
 __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, int EPI, int EPI2,
-                                          int N, int NP, int w0, int ncb, int t, float nrm,
-                                          MxShared s) {
+                                          int N, int M, Tile T, float nrm, MxShared s) {
   constexpr int NACC = K::NACC;
   const bool STACK = EPI2 >= 0;
-  const Tiles T = tiles_of<K>(N, NP, w0, ncb, STACK);
   const size_t NN = (size_t)N * N;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ks = t % T.nks, u = t / T.nks, cb = u % ncb;
-  const int rb0 = (u / ncb) * 128, jb = cb * w0, width = min(w0, NP - jb);
-  const bool first = ks == 0, last = ks == T.nks - 1;
+  const int rb0 = T.rb0, jb = T.jb, width = T.width;
+  const bool first = T.ka == 0, last = T.kb == N;
   const int quad = warp & 3, hw = warp >> 2;
   // a warp whose 32 tensor-memory lanes are all padding rows has nothing to drain
-  if (rb0 + quad * 32 >= T.M) return nrm;
+  if (rb0 + quad * 32 >= M) return nrm;
   const int row = rb0 + quad * 32 + lane;
   // the lower rows of a stacked product: their own epilogue and outputs
-  const bool live = row < T.M, upper = !STACK || row < N;
+  const bool live = row < M, upper = !STACK || row < N;
   const int epi = upper ? EPI : EPI2;
   const int rowL = upper ? row : row - N;
   const int ox = upper ? (op >> 8) & 15 : (op >> 20) & 15;
@@ -795,9 +865,10 @@ __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, 
   double2* const o1b = W + (upper ? (op >> 12) & 15 : (op >> 24) & 15) * NN + rowL;   // aux
   // column exponents of the outputs (a warp's rows may belong to both products)
   const int oU = (op >> 8) & 15, oL = (op >> 20) & 15;
-  int* const cU = (last && oU >= 3 && (!STACK || rb0 + quad * 32 < N)) ? s.cols(oU, N) : nullptr;
-  int* const cL = (last && STACK && oL >= 3 && rb0 + quad * 32 + 31 >= N) ? s.cols(oL, N) : nullptr;
-  int rmax = 0;
+  // (matrices 6 and 7, M1 and M2, are left factors only)
+  int* const cU = (last && oU >= 3 && oU != 6 && oU != 7 && (!STACK || rb0 + quad * 32 < N)) ? s.cols(oU, N) : nullptr;
+  int* const cL = (last && STACK && oL >= 3 && oL != 6 && oL != 7 && rb0 + quad * 32 + 31 >= N) ? s.cols(oL, N) : nullptr;
+  unsigned rmax = 0;                       // upper words without sign: ordered like exponents
   const uint32_t tq = s.t().tslot + ((uint32_t)(quad * 32) << 16);
   for (int cg = hw * 4; cg < width; cg += 16) {
 #pragma unroll 1
@@ -811,67 +882,102 @@ __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, 
           tmem_ld2(ta, v[comp][a]);
           ta += (uint32_t)width;
         }
-      double2 old0[2], old1[2];
-#pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {          // the epilogue's loads
-        const int j = jb + c0 + jj;
-        old0[jj] = make_double2(0.0, 0.0);
-        old1[jj] = old0[jj];
-        if (live && j < N) {
-          if (epi == OZ_ADD2) old1[jj] = o1b[(size_t)j * N];
-          if (epi == OZ_ADD2 || !first) old0[jj] = o0b[(size_t)j * N];
-          else if (epi == OZ_ADDTO) old0[jj] = o1b[(size_t)j * N];
-        }
+      const int j0 = jb + c0;
+      const bool on0 = live && j0 < N, on1 = live && j0 + 1 < N;
+      double2* const p0 = o0b + (size_t)j0 * N;
+      double2* const q0 = o1b + (size_t)j0 * N;
+      double2 old0[2], old1[2];                 // the epilogue's loads
+      old0[0] = old0[1] = old1[0] = old1[1] = make_double2(0.0, 0.0);
+      if (epi == OZ_ADD2 || epi == OZ_ADDTO) {
+        if (on0) old1[0] = q0[0];
+        if (on1) old1[1] = q0[N];
+      }
+      if (epi == OZ_ADD2 || !first) {
+        if (on0) old0[0] = p0[0];
+        if (on1) old0[1] = p0[N];
       }
       tmem_wait_ld();
+      double2 val[2];
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {          // without branches: four values in flight
+        const int ee = er + eY[min(j0 + jj, N - 1)];
+        uint32_t ar[NACC], ai[NACC];
+#pragma unroll
+        for (int a = 0; a < NACC; ++a) {
+          ar[a] = v[0][a][jj];
+          ai[a] = v[1][a][jj];
+        }
+        val[jj] = make_double2(K::value(ar, ee), K::value(ai, ee));
+      }
+      if (K::POISON) {
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj)
+          if (max(er, eY[min(j0 + jj, N - 1)]) == 2047) {
+            val[jj].x = __longlong_as_double(0x7FF8000000000000LL);
+            val[jj].y = val[jj].x;
+          }
+      }
+      if (epi == OZ_ADD2) {
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          old1[jj].x += val[jj].x;
+          old1[jj].y += val[jj].y;
+          val[jj].x += old0[jj].x;
+          val[jj].y += old0[jj].y;
+        }
+        if (on0) q0[0] = old1[0];
+        if (on1) q0[N] = old1[1];
+      } else if (epi == OZ_IMINUS) {
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          if (first) {
+            val[jj] = make_double2(-val[jj].x, -val[jj].y);
+            // (one of the warp's rows is on the diagonal; FP64 adds are not free: two a clock)
+            if ((unsigned)(j0 + jj - rb0 - quad * 32) < 32u && rowL == j0 + jj) val[jj].x += 1.0;
+          } else {
+            val[jj] = make_double2(old0[jj].x - val[jj].x, old0[jj].y - val[jj].y);
+          }
+        }
+      } else if (epi == OZ_ADDTO || !first) {
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          const double2 o = first ? old1[jj] : old0[jj];
+          val[jj].x += o.x;
+          val[jj].y += o.y;
+        }
+      }
+      if (on0) p0[0] = val[0];
+      if (on1) p0[N] = val[1];
+      if (last && (epi == OZ_STORE_NORM || epi == OZ_IMINUS)) {
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          if (!(jj ? on1 : on0)) continue;
+          const float fr = d2f_bits(val[jj].x), fi = d2f_bits(val[jj].y);
+          if (K::FRO && epi == OZ_IMINUS) nrm = fmaf(fr, fr, fmaf(fi, fi, nrm));
+          else nrm += fabsf(fr) + fabsf(fi);
+        }
+      }
+      unsigned e[2];
 #pragma unroll
       for (int jj = 0; jj < 2; ++jj) {
-        const int j = jb + c0 + jj;
-        int e = EXP_MIN;
-        if (live && j < N) {
-          const int ec = eY[j];
-          uint32_t ar[NACC], ai[NACC];
-#pragma unroll
-          for (int a = 0; a < NACC; ++a) {
-            ar[a] = v[0][a][jj];
-            ai[a] = v[1][a][jj];
-          }
-          double2 val = make_double2(K::value(ar, er + ec), K::value(ai, er + ec));
-          if (K::POISON && max(er, ec) == 2047) {
-            val.x = __longlong_as_double(0x7FF8000000000000LL);
-            val.y = val.x;
-          }
-          if (epi == OZ_ADD2) {
-            o1b[(size_t)j * N] = make_double2(old1[jj].x + val.x, old1[jj].y + val.y);
-            val = make_double2(old0[jj].x + val.x, old0[jj].y + val.y);
-          } else if (epi == OZ_IMINUS) {
-            if (first && rowL == j) old0[jj].x = 1.0;
-            if (first && rowL != j) val = make_double2(-val.x, -val.y);
-            else val = make_double2(old0[jj].x - val.x, old0[jj].y - val.y);
-          } else if (epi == OZ_ADDTO || !first) {
-            val = make_double2(old0[jj].x + val.x, old0[jj].y + val.y);
-          }
-          o0b[(size_t)j * N] = val;
-          if ((epi == OZ_STORE_NORM || epi == OZ_IMINUS) && last) {
-            const float fr = d2f_bits(val.x), fi = d2f_bits(val.y);
-            if (K::FRO && epi == OZ_IMINUS) nrm = fmaf(fr, fr, fmaf(fi, fi, nrm));
-            else nrm += fabsf(fr) + fabsf(fi);
-          }
-          e = max(bexp(val.x), bexp(val.y));
-        }
-        rmax = max(rmax, e);
-        if (cU) {
-          const int m = __reduce_max_sync(0xffffffffu, upper ? e : EXP_MIN);
-          if (lane == 0 && j < N) atomicMax(&cU[j], m);
-        }
-        if (cL) {
-          const int m = __reduce_max_sync(0xffffffffu, upper ? EXP_MIN : e);
-          if (lane == 0 && j < N) atomicMax(&cL[j], m);
-        }
+        e[jj] = max((unsigned)__double2hiint(val[jj].x) & 0x7FFFFFFFu,
+                    (unsigned)__double2hiint(val[jj].y) & 0x7FFFFFFFu);
+        if (!(jj ? on1 : on0)) e[jj] = 0;
+        rmax = max(rmax, e[jj]);
+      }
+      if (cU) {
+        const unsigned m0 = __reduce_max_sync(0xffffffffu, upper ? e[0] : 0u);
+        const unsigned m1 = __reduce_max_sync(0xffffffffu, upper ? e[1] : 0u);
+        if (lane < 2 && j0 + lane < N) atomicMax(&cU[j0 + lane], (int)((lane ? m1 : m0) >> 20));
+      }
+      if (cL) {
+        const unsigned m0 = __reduce_max_sync(0xffffffffu, upper ? 0u : e[0]);
+        const unsigned m1 = __reduce_max_sync(0xffffffffu, upper ? 0u : e[1]);
+        if (lane < 2 && j0 + lane < N) atomicMax(&cL[j0 + lane], (int)((lane ? m1 : m0) >> 20));
       }
     }
   }
-  if (last && ox >= 3 && live) atomicMax(&s.rows(ox, N)[rowL], rmax);
+  if (last && ox >= 3 && live) atomicMax(&s.rows(ox, N)[rowL], (int)(rmax >> 20));
   return nrm;
 }
 
@@ -884,10 +990,11 @@ __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, 
 template <class K>
 __device__ __noinline__ float split_gemm(double2* __restrict__ const W, const uint32_t op,
                                          const int EPI, const int EPI2, const int N, const int NP,
-                                         const int w0, const int ncb, const MxShared s) {
+                                         const int w0, const MxShared s) {
   SplitTail& sh = s.t();
   const int tid = threadIdx.x, warp = tid >> 5;
-  const Tiles T = tiles_of<K>(N, NP, w0, ncb, EPI2 >= 0);
+  const int M = EPI2 >= 0 ? 2 * N : N;           // rows of the tiles that hold outputs
+  const int kper = k_part<K>(N);
   const int oU = (op >> 8) & 15, oL = (op >> 20) & 15;
   float nrm = 0.f;
   // the outputs' exponents start at the floor
@@ -898,16 +1005,17 @@ __device__ __noinline__ float split_gemm(double2* __restrict__ const W, const ui
   __syncthreads();
   int abort = sh.abort;
   uint32_t c0 = sh.chunk;                        // first chunk of the tile
-  const int ntile = T.count();
   int ahead = 0;                                 // chunks of the tile generated already
-  for (int t = 0; t < ntile && !abort; ++t) {
-    const int nch = T.chunks(t % T.nks);
+  Tile T = first_tile(N, NP, w0, kper);
+  for (bool more = true; more && !abort;) {
+    const Tile C = T;                            // the current tile; T: the next one
+    const int nch = C.chunks();
+    more = next_tile(T, M, N, NP, w0, kper);
     if (warp == 0) {
       // one thread issues the tile's MMAs as its chunks become complete
       int ab = 0;
       if (elect_one()) {
-        const int width = min(w0, NP - (t / T.nks) % ncb * w0);
-        const int slot = K::SLOT + (width == w0 ? 0 : 1);
+        const int slot = K::SLOT + (C.width == w0 ? 0 : 1);
         const IssueTab* const tab = sh.tabs + slot;
         const int n = sh.ntab[slot];
         const uint32_t tmem = sh.tslot;
@@ -918,7 +1026,7 @@ __device__ __noinline__ float split_gemm(double2* __restrict__ const W, const ui
             break;
           }
           tc_fence_after();
-          split_issue<K>(tab, n, saddr(s.base()) + (q & 1) * s.stage, tmem, width, c > 0);
+          split_issue<K>(tab, n, saddr(s.base()) + (q & 1) * s.stage, tmem, C.width, c > 0);
           mma_commit(&sh.empty[q & 1]);
           sh.issued = q + 1;
         }
@@ -927,11 +1035,10 @@ __device__ __noinline__ float split_gemm(double2* __restrict__ const W, const ui
       abort |= __any_sync(0xffffffffu, ab);
     } else {
       // this tile's chunks and the first two of the next one
-      if (ahead < nch)
-        abort |= split_generate<K>(W, op, N, NP, w0, ncb, EPI2 >= 0, t, ahead, nch, c0 + ahead, s);
-      if (t + 1 < ntile && !abort) {
-        ahead = min(2, T.chunks((t + 1) % T.nks));
-        abort |= split_generate<K>(W, op, N, NP, w0, ncb, EPI2 >= 0, t + 1, 0, ahead, c0 + nch, s);
+      if (ahead < nch) abort |= split_generate<K>(W, op, N, M, C, ahead, nch, c0 + ahead, s);
+      if (more && !abort) {
+        ahead = min(2, T.chunks());
+        abort |= split_generate<K>(W, op, N, M, T, 0, ahead, c0 + nch, s);
       }
     }
     // all MMAs of this tile: the last commit covers every earlier one
@@ -941,7 +1048,7 @@ __device__ __noinline__ float split_gemm(double2* __restrict__ const W, const ui
     __syncwarp();
     if (!__any_sync(0xffffffffu, abort)) {
       tc_fence_after();
-      nrm = split_drain<K>(W, op, EPI, EPI2, N, NP, w0, ncb, t, nrm, s);
+      nrm = split_drain<K>(W, op, EPI, EPI2, N, M, C, nrm, s);
     }
     tc_fence_before();
     abort = __syncthreads_or(abort);

@@ -41,12 +41,12 @@ __host__ __device__ inline MxPlan s64_plan(int N) { return split_plan(N, split_w
 
 __device__ __forceinline__ float gemm7(double2* W, uint32_t op, int epi, int epi2, const MxPlan& p,
                                        const MxShared s) {
-  return split_gemm<Dig7>(W, op, epi, epi2, p.N, p.NP, p.w0, p.ncb, s);
+  return split_gemm<Dig7>(W, op, epi, epi2, p.N, p.NP, p.w0, s);
 }
 __device__ __forceinline__ void gemm4(double2* W, uint32_t op, int epi, const MxPlan& p7,
                                       const MxShared s) {
   const MxPlan p = split_plan4(p7);
-  split_gemm<Dig4>(W, op, epi, -1, p.N, p.NP, p.w0, p.ncb, s);
+  split_gemm<Dig4>(W, op, epi, -1, p.N, p.NP, p.w0, s);
 }
 
 // the FP64 Gauss-Jordan of the plain form, un-permuted into dst; its area
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(SP_T, 1) k_split64_unit(int op, int N, double2
     for (int e = tid; e < NN; e += blockDim.x) negX[e] = make_double2(-W[e].x, -W[e].y);
     __syncthreads();
     int G = 3, Gn = 4;
-    sing = s64_inverse(7, make_double2(0.0, 0.0), W, pl, G, Gn, 5, 6, -1, -1, 0, s);
+    sing = s64_inverse(7, make_double2(0.0, 0.0), W, pl, G, Gn, 6, 5, -1, -1, 0, s);
     __syncthreads();
     double2* C = W + 2 * (size_t)NN;
     for (int e = tid; e < NN; e += blockDim.x) C[e] = W[(size_t)G * NN + e];
