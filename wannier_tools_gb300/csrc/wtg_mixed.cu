@@ -12,7 +12,7 @@
 // above) followed by Newton-Schulz refinement X <- X + X (I - M X): the
 // residual I - M X is a 7-digit split product, the correction X R a 4-digit
 // one (R is small).  The three final inverses (src/surfgreen.f90:127-134) are
-// FP64 Gauss-Jordan (the FP64 form's own code), and the convergence test
+// FP64 (the FP64 form's own), and the convergence test
 // sum |alpha_ij| (src/surfgreen.f90:120) takes each |alpha_ij| and the sum in
 // FP64 wherever the FP32 bounds of the sum do not decide it.
 #include <mutex>
@@ -26,6 +26,7 @@ namespace {
 
 #include "wtg_fp64_dev.cuh"
 #include "wtg_split.cuh"
+#include "wtg_split_inverse.cuh"
 
 // 7-digit products, and the 4-digit corrections of the refinement
 using Dig7 = DigB7<7>;
@@ -80,20 +81,14 @@ __device__ int mixed_inverse(const double2* X, double2 w, double2* W, const MxPl
 // iterations, status) in thread 0, the final inverses to gll / grr / gb when
 // those are not null.  o has DecimArgs' member names (lists, tolerance, ...).
 // The loop's products and inverses are the split-BF16 forms; the three final
-// inverses (src/surfgreen.f90:127-134) are FP64 Gauss-Jordan, the FP64 form's
-// own (gj_invert in shared memory up to MX_SMEM_GJ_N, gj_invert_global in
-// workspace matrix 8 above), in an area that aliases the idle operand buffers.
+// inverses (src/surfgreen.f90:127-134) are FP64 (split_finals).
 template <class O, class Emit>
 __device__ __forceinline__ void mixed_solve(const MxPlan& pl, double2 w, const O& o, int ns_iter,
                                             double2* gll, double2* grr, double2* gb, double2* W,
                                             const MxShared s, Emit emit) {
   const int N = pl.N, NN = N * N, tid = threadIdx.x;
-  double2* E = W;
-  double2* ES = W + (size_t)NN;
-  double2* ET = W + (size_t)2 * NN;
   int Al = 3, Be = 4, G = 5, R = 9, Gn = 10;         // workspace matrices by index
   constexpr int iE = 0, iES = 1, iET = 2, M1 = 6, M2 = 7, iMi = 8;
-  double2* const Mi = W + (size_t)iMi * NN;
   int stat = 0, it = 0;
   bool conv = false;
   split_tables<Dig7, Dig4>(pl, s);
@@ -103,7 +98,7 @@ __device__ __forceinline__ void mixed_solve(const MxPlan& pl, double2 w, const O
     it = itc;
     // the refinement stops at a residual sum of 1e-4 Ndim (then ~1e-8 after its
     // update): the dense Fermi-arc check stays below 2e-6 against the FP64 oracle
-    if (mixed_inverse(E, w, W, pl, ns_iter, G, Gn, iMi, R, s, 1e-4f)) stat |= PT_SINGULAR;
+    if (mixed_inverse(W, w, W, pl, ns_iter, G, Gn, iMi, R, s, 1e-4f)) stat |= PT_SINGULAR;
     // the reference's six products (:92-116); eps still receives M1 beta before
     // M2 alpha.  Where it takes fewer 128-row tiles (Ndim mod 128 in 1..64: up to
     // Ndim 64, or 129..192, 257..320), the products with a common right factor
@@ -131,83 +126,18 @@ __device__ __forceinline__ void mixed_solve(const MxPlan& pl, double2 w, const O
   }
   if (!conv) stat |= PT_NOT_CONVERGED;
 
-  extern __shared__ __align__(1024) unsigned char smem_dyn[];
-  const bool gsm = N <= MX_SMEM_GJ_N;
-  const Shared fs = fp64_layout(smem_dyn, N, GJ_PANEL, gsm);
-  // (w - X)^-1 in FP64, optionally stored un-permuted to dst; ginv reads the
-  // result.  blk 1 / 2: only the leading / trailing nw x nw block (one principal
-  // layer), by the Schur complement of the rest (schur_block_invert), where the
-  // spectral sums read nothing else; a zero pivot there takes the full inverse.
-  const int m = N - o.nw;
-  // above MX_SMEM_GJ_N the elimination runs in workspace matrix 8 and the
-  // block's inverse in shared memory, when the block fits the area
-  const bool gblk = !gsm && schur_area_bytes(N, o.nw) <= MX_FP64_AREA;
-  const Shared fb = schur_layout(smem_dyn, N, o.nw);
-  int blk = 0;
-  auto invert = [&](const double2* X, double2* dst, int want_blk) -> int {
-    __syncthreads();                  // the area aliases buffers the loop just used
-    blk = ((gsm || gblk) && !dst && m > 0) ? want_blk : 0;
-    if (blk && !(gsm ? schur_block_invert(X, w, N, o.nw, blk == 1, fs)
-                     : schur_block_invert_global(X, w, N, o.nw, blk == 1, Mi, fb)))
-      return 0;
-    blk = 0;
-    int sing;
-    if (gsm) {
-      sing = gj_invert(X, w, N, fs);
-      if (dst) gj_store(N, fs, dst);
-    } else {
-      sing = gj_invert_global(X, w, N, Mi, fs);
-      if (dst) gj_store_global(N, Mi, fs, dst);
-    }
-    return sing;
-  };
-  auto ginv = [&](int i, int j) {
-    if (blk) {                        // block entry (i, j): local indices in the block
-      const int li = blk == 1 ? o.nw - 1 - i : i - m;
-      const int lj = blk == 1 ? o.nw - 1 - j : j - m;
-      return gsm ? fs.big[m + li + (size_t)(m + fs.cols[lj]) * N]
-                 : fb.big[li + (size_t)fb.cols[lj] * o.nw];
-    }
-    return gsm ? fs.big[i + fs.cols[j] * N] : Mi[i + (size_t)fs.cols[j] * N];
-  };
-  double dl = 0.0, dr = 0.0, db = 0.0;
-  double spin[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  if (invert(ES, gll, 1)) stat |= PT_SINGULAR;                // :127-128
+  // the three final inverses in FP64, refined on 55-bit products (Ndim 112:
+  // eliminations on the FP64 pipe took 17 % of a solve, 112 against 103.5 ms for 912
+  // points; Ndim 40: 64.4 and 65.9 ms for 5151)
+  MxPlan pf = split_plan(N, min(split_wmax<F8x7>(), pl.wb));
+  pf.wb = pl.wb;
+  split_tables<F8x7, F8x4>(pf, s);
+  double sums[9];                                   // dl, dr, db, then the six spin sums
+  if (split_finals(w, W, pf, o, G, Gn, iMi, R, gll, grr, gb, 0, sums, s)) stat |= PT_SINGULAR;
   if (tid == 0) {
-    for (int q = 0; q < o.ntop; ++q) {
-      const int io = o.top[q] - 1;
-      const double v = ginv(io, io).y;
-      dl = o.divide_by_pi ? dl - v / PI_REF : dl - v;
-    }
-    if (o.spin[0]) spin_sums(ginv, o.nw, o.ntop, o.top, 0, o.divide_by_pi, spin[0], spin[1], spin[2]);
-  }
-  __syncthreads();
-  // surfstat's spin sums read GRR's leading block as well (src/surfstat.f90:178-192)
-  if (invert(ET, grr, (o.spin[0] && !o.spin_right_bottom) ? 0 : 2))    // :130-131
-    stat |= PT_SINGULAR;
-  if (tid == 0) {
-    for (int q = 0; q < o.nbot; ++q) {
-      const int io = N - o.nw + o.bot[q] - 1;
-      const double v = ginv(io, io).y;
-      dr = o.divide_by_pi ? dr - v / PI_REF : dr - v;
-    }
-    if (o.spin[0]) {
-      if (o.spin_right_bottom)
-        spin_sums(ginv, o.nw, o.nbot, o.bot, N - o.nw, o.divide_by_pi, spin[3], spin[4], spin[5]);
-      else
-        spin_sums(ginv, o.nw, o.ntop, o.top, 0, o.divide_by_pi, spin[3], spin[4], spin[5]);
-    }
-  }
-  __syncthreads();
-  if (invert(E, gb, 0)) stat |= PT_SINGULAR;                  // :133-134
-  if (tid == 0) {
-    for (int i = 0; i < N; ++i) {
-      const double v = ginv(i, i).y;
-      db = o.divide_by_pi ? db - v / PI_REF : db - v;
-    }
     if (s.t().abort) stat |= PT_TIMEOUT;
-    if (!isfinite(dl) || !isfinite(dr) || !isfinite(db)) stat |= PT_NONFINITE;
-    emit(dl, dr, db, spin, it, stat);
+    if (!isfinite(sums[0]) || !isfinite(sums[1]) || !isfinite(sums[2])) stat |= PT_NONFINITE;
+    emit(sums[0], sums[1], sums[2], sums + 3, it, stat);
   }
   __syncthreads();
 }

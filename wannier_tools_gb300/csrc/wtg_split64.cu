@@ -32,111 +32,8 @@ namespace {
 
 #include "wtg_fp64_dev.cuh"
 #include "wtg_split.cuh"
+#include "wtg_split_inverse.cuh"
 #include "wtg_fp64_solve.cuh"
-
-using Dig7 = DigF8<7>;
-using Dig4 = DigF8<4>;
-
-__host__ __device__ inline MxPlan s64_plan(int N) { return split_plan(N, split_wmax<Dig7>()); }
-
-__device__ __forceinline__ float gemm7(double2* W, uint32_t op, int epi, int epi2, const MxPlan& p,
-                                       const MxShared s) {
-  return split_gemm<Dig7>(W, op, epi, epi2, p.N, p.NP, p.w0, s);
-}
-__device__ __forceinline__ void gemm4(double2* W, uint32_t op, int epi, const MxPlan& p7,
-                                      const MxShared s) {
-  const MxPlan p = split_plan4(p7);
-  split_gemm<Dig4>(W, op, epi, -1, p.N, p.NP, p.w0, s);
-}
-
-// the FP64 Gauss-Jordan of the plain form, un-permuted into dst; its area
-// aliases the stages and the exponents.  Mg: work for the global-memory variant.
-__device__ __noinline__ int gj64(const double2* X, double2 w, int N, double2* dst, double2* Mg,
-                                 int gi) {
-  extern __shared__ __align__(1024) unsigned char smem_dyn[];
-  const bool gsm = N <= MX_SMEM_GJ_N && !gi;
-  const Shared fs = fp64_layout(smem_dyn, N, GJ_PANEL, gsm);
-  __syncthreads();
-  int sing;
-  if (gsm) {
-    sing = gj_invert(X, w, N, fs);
-    gj_store(N, fs, dst);
-  } else {
-    sing = gj_invert_global(X, w, N, Mg, fs);
-    gj_store_global(N, Mg, fs, dst);
-  }
-  __syncthreads();
-  return sing;
-}
-
-// (w I - W[iX])^-1 into workspace matrix G with its exponents (see the head of
-// the file).  Uses matrices Mi, R, Gn as work; swaps G and Gn.  live0 / live1:
-// matrices whose exponents a fallback has to make again (-1: none).
-__device__ int s64_inverse(int iX, double2 w, double2* W, const MxPlan& pl, int& G, int& Gn, int Mi,
-                           int R, int live0, int live1, int gi, const MxShared s) {
-  const int N = pl.N;
-  const size_t NN = (size_t)N * N;
-  bool good = false;
-  if (!gj32(W + iX * NN, w, N, W, Mi, G, R, s)) {
-    float prev = 3.0e38f;
-    for (int t = 0; t < 8 && !s.t().abort; ++t) {
-      // R = I - M G; the sum is |R|_F^2
-      const float res = sqrtf(block_sum_f(gemm7(W, ops(Mi, G, R), OZ_IMINUS, -1, pl, s), s));
-      if (!(res < 0.25f * prev)) break;               // no longer converging (or NaN)
-      // Gn = G + G R: 30 bits of R keep the step's own error below |R| 2^-30
-      gemm4(W, ops(G, R, Gn, G), OZ_ADDTO, pl, s);
-      swap_mat(G, Gn);
-      if (res <= 1e-8f) {                             // the step left at most 1e-16
-        good = true;
-        break;
-      }
-      prev = res;
-    }
-  }
-  if (good || s.t().abort) return 0;
-  const int sing = gj64(W + iX * NN, w, N, W + G * NN, W + Mi * NN, gi);
-  exps_of(W + G * NN, G, N, s);
-  if (live0 >= 0) exps_of(W + live0 * NN, live0, N, s);
-  if (live1 >= 0) exps_of(W + live1 * NN, live1, N, s);
-  return sing;
-}
-
-// sum over q = 0 .. n-1 of f(q), subtracted term by term in order (as the
-// reference's loops), the terms evaluated by all threads; result in thread 0
-template <class F>
-__device__ double list_sum(int n, F f, const MxShared s) {
-  double* buf = reinterpret_cast<double*>(s.base());
-  constexpr int NB = 4096;
-  double acc = 0.0;
-  for (int q0 = 0; q0 < n; q0 += NB) {
-    const int m = min(NB, n - q0);
-    __syncthreads();
-    for (int q = threadIdx.x; q < m; q += blockDim.x) buf[q] = f(q0 + q);
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int q = 0; q < m; ++q) acc = acc - buf[q];
-  }
-  __syncthreads();
-  return acc;
-}
-
-// spin terms of orbital io (1-based list entry + offset - 1): see spin_sums
-__device__ __forceinline__ double spin_term(const double2* G, int N, int nw, int io, int c) {
-  const int nwh = nw / 2, jl = io % nw;
-  int partner = -1;
-  double sgn = 0.0;
-  if (jl < nwh) {
-    partner = io + nwh;
-    sgn = 1.0;
-  } else if (jl < 2 * nwh) {
-    partner = io - nwh;
-    sgn = -1.0;
-  }
-  if (partner < 0) return 0.0;
-  if (c == 2) return sgn * G[io + (size_t)io * N].y;
-  const double2 gp = G[io + (size_t)partner * N];
-  return c == 0 ? gp.y : sgn * gp.x;
-}
 
 // Decimation of one instance whose eps, eps_s, eps_t (= H00), alpha (= H01) and
 // beta (= H01^dagger) already sit in workspace matrices 0..4 of W (11 N x N
@@ -150,7 +47,7 @@ __device__ __forceinline__ void s64_solve(const MxPlan& pl, double2 w, const O& 
   constexpr int iE = 0, iES = 1, iET = 2, M1 = 6, M2 = 7, iMi = 8;
   int stat = 0, it = 0;
   bool conv = false;
-  split_tables<Dig7, Dig4>(pl, s);
+  split_tables<F8x7, F8x4>(pl, s);
   exps_of(W + (size_t)Al * NN, Al, N, s);
   exps_dagger(Be, Al, N, s);
   for (int itc = 1; itc <= o.itermax && !s.t().abort; ++itc) {   // src/surfgreen.f90:86-122
@@ -160,16 +57,16 @@ __device__ __forceinline__ void s64_solve(const MxPlan& pl, double2 w, const O& 
     // tiles; eps still receives M1 beta before M2 alpha
     float part;
     if ((2 * N + 127) / 128 < 2 * ((N + 127) / 128)) {
-      gemm7(W, ops(Al, G, M1, 0, Be, M2), OZ_STORE, OZ_STORE, pl, s);               // :92, :95
-      gemm7(W, ops(M1, Be, iE, iES, M2, R), OZ_ADD2, OZ_STORE, pl, s);              // :98-102, :116
-      part = gemm7(W, ops(M1, Al, Gn, 0, M2, iE, iET), OZ_STORE_NORM, OZ_ADD2, pl, s);  // :113, :107-110
+      f8_gemm7(W, ops(Al, G, M1, 0, Be, M2), OZ_STORE, OZ_STORE, pl, s);               // :92, :95
+      f8_gemm7(W, ops(M1, Be, iE, iES, M2, R), OZ_ADD2, OZ_STORE, pl, s);              // :98-102, :116
+      part = f8_gemm7(W, ops(M1, Al, Gn, 0, M2, iE, iET), OZ_STORE_NORM, OZ_ADD2, pl, s);  // :113, :107-110
     } else {
-      gemm7(W, ops(Al, G, M1), OZ_STORE, -1, pl, s);                                // :92
-      gemm7(W, ops(Be, G, M2), OZ_STORE, -1, pl, s);                                // :95
-      gemm7(W, ops(M1, Be, iE, iES), OZ_ADD2, -1, pl, s);                           // :98-102
-      part = gemm7(W, ops(M1, Al, Gn), OZ_STORE_NORM, -1, pl, s);                   // :113
-      gemm7(W, ops(M2, Al, iE, iET), OZ_ADD2, -1, pl, s);                           // :107-110
-      gemm7(W, ops(M2, Be, R), OZ_STORE, -1, pl, s);                                // :116
+      f8_gemm7(W, ops(Al, G, M1), OZ_STORE, -1, pl, s);                                // :92
+      f8_gemm7(W, ops(Be, G, M2), OZ_STORE, -1, pl, s);                                // :95
+      f8_gemm7(W, ops(M1, Be, iE, iES), OZ_ADD2, -1, pl, s);                           // :98-102
+      part = f8_gemm7(W, ops(M1, Al, Gn), OZ_STORE_NORM, -1, pl, s);                   // :113
+      f8_gemm7(W, ops(M2, Al, iE, iET), OZ_ADD2, -1, pl, s);                           // :107-110
+      f8_gemm7(W, ops(M2, Be, R), OZ_STORE, -1, pl, s);                                // :116
     }
     swap_mat(Al, Gn);
     swap_mat(Be, R);
@@ -180,35 +77,8 @@ __device__ __forceinline__ void s64_solve(const MxPlan& pl, double2 w, const O& 
   }
   if (!conv) stat |= PT_NOT_CONVERGED;
 
-  // GLL = (w - eps_s)^-1, GRR = (w - eps_t)^-1, GB = (w - eps)^-1   // :127-134
   double sums[9];                                   // dl, dr, db, then the six spin sums
-  for (int k = 0; k < 3; ++k) {
-    const int iX = k == 0 ? iES : k == 1 ? iET : iE;
-    double2* const dst = k == 0 ? gll : k == 1 ? grr : gb;
-    if (s64_inverse(iX, w, W, pl, G, Gn, iMi, R, -1, -1, gi, s)) stat |= PT_SINGULAR;
-    __syncthreads();
-    const double2* const g = W + (size_t)G * NN;
-    if (dst)
-      for (int e = tid; e < NN; e += blockDim.x) dst[e] = g[e];
-    const int n = k == 0 ? o.ntop : k == 1 ? o.nbot : N;
-    auto idx = [&](int q) {
-      return k == 0 ? o.top[q] - 1 : k == 1 ? N - o.nw + o.bot[q] - 1 : q;
-    };
-    auto scaled = [&](double v) { return o.divide_by_pi ? v / PI_REF : v; };
-    sums[k] = list_sum(n, [&](int q) {
-      const int io = idx(q);
-      return scaled(g[io + (size_t)io * N].y);
-    }, s);
-    if (k < 2 && o.spin[0]) {                       // src/surfstat.f90:162-192
-      // surfstat's right sums run over the top list (as the reference's do)
-      const bool top = k == 0 || !o.spin_right_bottom;
-      const int off = top ? 0 : N - o.nw;
-      for (int c = 0; c < 3; ++c)
-        sums[3 + 3 * k + c] = list_sum(top ? o.ntop : o.nbot, [&](int q) {
-          return scaled(spin_term(g, N, o.nw, off + (top ? o.top[q] : o.bot[q]) - 1, c));
-        }, s);
-    }
-  }
+  if (split_finals(w, W, pl, o, G, Gn, iMi, R, gll, grr, gb, gi, sums, s)) stat |= PT_SINGULAR;
   if (tid == 0) {
     if (s.t().abort) stat |= PT_TIMEOUT;
     if (!isfinite(sums[0]) || !isfinite(sums[1]) || !isfinite(sums[2])) stat |= PT_NONFINITE;
@@ -352,12 +222,12 @@ __global__ void __launch_bounds__(SP_T, 1) k_split64_unit(int op, int N, double2
   const int NN = N * N, tid = threadIdx.x;
   const MxShared s = mx_layout(pl.wb);
   mx_setup(s, 0u);
-  split_tables<Dig7, Dig4>(pl, s);
+  split_tables<F8x7, F8x4>(pl, s);
   int sing = 0;
   if (op == 0) {
     exps_of(W, 0, N, s);
     exps_of(W + NN, 1, N, s);
-    gemm7(W, ops(0, 1, 2), OZ_STORE, -1, pl, s);
+    f8_gemm7(W, ops(0, 1, 2), OZ_STORE, -1, pl, s);
   } else {
     // C = X^-1: X given directly, so pass -X with w = 0 (M = 0*I - (-X) = X)
     double2* negX = W + 7 * (size_t)NN;
