@@ -139,17 +139,17 @@ int run_spectrum(wtg_model* m, int nk, const double* d_k, int nomega, const doub
                                       (mixed ? "mixed" : "FP64") + " kernel limit " +
                                       std::to_string(nmax));
   wtg::DecimConfig cfg;
+  int nsm = 0;
+  WTG_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device));
   if (mixed) {
     WTG_CK(wtg::decim_mixed_config(N, &cfg));
   } else {
     // the large-Ndim (global-memory inverse) variant at any Ndim when a test asks for it
-    WTG_CK(wtg::decim_fp64_config(N, 0, &cfg,
+    WTG_CK(wtg::decim_fp64_config(N, wtg::fp64_threads_for(N, (long long)nk * nomega, nsm), &cfg,
                                   wtg::test_option(WTG_TEST_FP64_GLOBAL_INVERSE) != 0));
   }
   const size_t ws_mats = mixed ? wtg::decim_mixed_ws_matrices() : wtg::decim_fp64_ws_matrices(cfg);
   if (cfg.ctas_per_sm < 1) return fail(WTG_EUNSUPPORTED, "decimation kernel does not fit an SM");
-  int nsm = 0;
-  WTG_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device));
 
   const size_t hk = sizeof(double2) * 2 * (size_t)N * N;   // H00+H01 per k
   const int grid_max = cfg.ctas_per_sm * nsm;
@@ -777,7 +777,7 @@ int wtg_surfgreen_1985(int ndim, double omega, double eta, const double* h00, co
     return fail(WTG_ENODEV, "no CUDA device available");
   const size_t nn = (size_t)ndim * ndim;
   wtg::DecimConfig cfg;
-  WTG_CK(wtg::decim_fp64_config(ndim, 0, &cfg));
+  WTG_CK(wtg::decim_fp64_config(ndim, 0, &cfg, false, true));
   // one allocation: h[2nn] | gll grr gb [3nn] | ws [8, 9 or 11 nn] | omega | outputs
   const size_t wsm = wtg::decim_fp64_ws_matrices(cfg);
   const size_t bytes = sizeof(double2) * ((5 + wsm) * nn) + 64 + 64;

@@ -179,12 +179,15 @@ struct DecimConfig {
   int ctas_per_sm;
   int inv_global = 0;         // FP64: 1 = the inverse runs in global memory (large Ndim)
   int w0 = 0;                 // mixed: output-column pass width
+  int small = 0;              // FP64: lanes of a warp per instance, no workspace
   int split = 0;              // products on the tensor cores (mixed form; FP64 form's split kernel)
 };
 
 // Built-in choices and limits of the tunable shapes, and the mixed form's pass
 // width for Ndim N after the tile table.
 int fp64_threads_default(int N);
+// threads per CTA of the FP64 pipe kernel for a launch of n_inst instances
+int fp64_threads_for(int N, long long n_inst, int nsm);
 int mixed_w0_default(int N);
 int mixed_w0_max(int N);
 int batch_mixed_w0(int N);
@@ -210,7 +213,7 @@ size_t decim_fp64_ws_matrices(const DecimConfig& cfg);
 // runs in global memory above decim_fp64_max_n(), or at any N with force_global (the two
 // variants agree bit for bit).
 cudaError_t decim_fp64_config(int N, int threads_override, DecimConfig* cfg,
-                              bool force_global = false);
+                              bool force_global = false, bool full_out = false);
 cudaError_t launch_decimate_fp64(const DecimArgs& a, const DecimConfig& cfg, int grid,
                                  cudaStream_t s);
 
@@ -223,13 +226,15 @@ cudaError_t launch_decimate_mixed(const DecimArgs& a, const DecimConfig& cfg, in
                                   cudaStream_t s);
 
 // The FP64 form on exactly split tensor-core products (wtg_split64.cu) runs in
-// this range of Ndim.  Below it a product fills too little of a 128-row tile.
+// this range of Ndim.  Below it a product fills too little of a 128-row tile
+// (5 000 points at Ndim 24: 44.3 ms on the FP64 pipe, 44.8 split; 3 148 at 28:
+// 45.5 and 31.6).
 // Above it the form stays on the FP64 pipe: its results there (Ndim 264, eta
 // 1e-3 eV) are compared to 1e-9 with FP64 evaluations that are themselves up to
 // 2e-9 off (80-bit evaluation of the same points; the split kernel is within
 // 2e-10 of it, the FP64 pipe within 9e-10), so only the plain operations agree
 // with them everywhere.
-constexpr int FP64_SPLIT_MIN_N = 33;
+constexpr int FP64_SPLIT_MIN_N = 25;
 constexpr int FP64_SPLIT_MAX_N = 256;
 constexpr bool fp64_split(int N) { return N >= FP64_SPLIT_MIN_N && N <= FP64_SPLIT_MAX_N; }
 cudaError_t split64_config(int N, DecimConfig* cfg);

@@ -34,6 +34,7 @@ namespace {
 #include "wtg_fp64_dev.cuh"
 
 #include "wtg_fp64_solve.cuh"
+#include "wtg_small_dev.cuh"
 
 template <int RP, bool GI>
 __global__ void __launch_bounds__(GI ? 256 : 512, 1) k_decimate_fp64(const __grid_constant__ DecimArgs a) {
@@ -76,6 +77,35 @@ __global__ void __launch_bounds__(GI ? 256 : 512, 1) k_decimate_fp64(const __gri
                          if (a.iters) a.iters[oidx] = it;
                          if (a.status) a.status[oidx] = (uint8_t)st;
                        });
+  }
+}
+
+// Ndim <= 8: a group of lanes per instance (small_solve), warps striding over the
+// instances
+template <int P>
+__global__ void __launch_bounds__(128) k_decimate_small(const __grid_constant__ DecimArgs a) {
+  constexpr int PER = 32 / Small<P>::G;            // instances a warp
+  const int N = a.N, NN = N * N;
+  const long long nwarp = (long long)gridDim.x * 4;
+  const int sub = (threadIdx.x & 31) / Small<P>::G;
+  for (long long q = ((long long)blockIdx.x * 4 + (threadIdx.x >> 5)) * PER; q < a.n_inst;
+       q += nwarp * PER) {
+    const bool valid = q + sub < a.n_inst;
+    const int inst = valid ? (int)(q + sub) : 0;
+    const int ik = inst / a.nomega, iw = inst % a.nomega;
+    const double2* H00 = a.h + (size_t)ik * 2 * NN;
+    const double2 w = make_double2(a.omega[iw], a.eta);     // src/surfgreen.f90:82
+    const size_t oidx = (size_t)(a.k_offset + ik) + (size_t)iw * a.nk_total;
+    small_solve<P>(N, w, a, H00, H00 + NN, valid,
+                   [&](double dl, double dr, double db, const double* spin, int it, int st) {
+                     a.dos_l[oidx] = dl;
+                     a.dos_r[oidx] = dr;
+                     a.dos_bulk[oidx] = db;
+                     if (a.spin[0])
+                       for (int c = 0; c < 6; ++c) a.spin[c][oidx] = spin[c];
+                     if (a.iters) a.iters[oidx] = it;
+                     if (a.status) a.status[oidx] = (uint8_t)st;
+                   });
   }
 }
 
@@ -125,7 +155,10 @@ __global__ void __launch_bounds__(256, 1) k_batch_fp64(const __grid_constant__ B
       if (a.iters) a.iters[p] = it;
       if (a.status) a.status[p] = (uint8_t)st;
     };
-    if (gi) fp64_solve<13, true>(N, a.KC, w, o, nullptr, nullptr, nullptr, W, s, emit);
+    if (N <= SMALL_MAX_N) {                  // one warp, as k_decimate_small
+      if (tid < 32) small_point(N, w, o, W, emit);
+      __syncthreads();
+    } else if (gi) fp64_solve<13, true>(N, a.KC, w, o, nullptr, nullptr, nullptr, W, s, emit);
     else fp64_solve<13, false>(N, a.KC, w, o, nullptr, nullptr, nullptr, W, s, emit);
   }
 }
@@ -174,8 +207,21 @@ int decim_fp64_large_max_n() { return 32 * GJ_ROWS; }
 
 int fp64_threads_default(int N) { return N <= 48 ? 128 : (N <= 80 ? 256 : 512); }
 
+int fp64_threads_for(int N, long long n_inst, int nsm) {
+  const int tile = tile_value(0, N);
+  if (tile > 0) return tile;
+  // from timings at Ndim 12 / 16 / 20 / 24: with no more instances than SMs a wider
+  // CTA shortens each (0.77 -> 0.67, 0.95 -> 0.85, 1.94 -> 1.52, 2.33 -> 2.15 ms a
+  // point against 128 threads); with many, narrow ones keep more instances in
+  // flight (20 000, 16 875 and 8 639 points: 38.6 -> 32.1, 43.5 -> 43.3, 52.5 ->
+  // 46.7 ms with 64 threads)
+  if (N >= 12 && N <= 32 && n_inst <= nsm) return 256;
+  if (N <= 20 && n_inst >= 8LL * nsm) return 64;
+  return fp64_threads_default(N);
+}
+
 size_t decim_fp64_ws_matrices(const DecimConfig& cfg) {
-  return cfg.split ? 11 : cfg.inv_global ? 9 : 8;
+  return cfg.small ? 0 : cfg.split ? 11 : cfg.inv_global ? 9 : 8;
 }
 
 // launch shape of the kernel on the FP64 pipe
@@ -218,7 +264,19 @@ static cudaError_t dfma_config(int N, int threads_override, DecimConfig* cfg, bo
   return cudaSuccess;
 }
 
-cudaError_t decim_fp64_config(int N, int threads_override, DecimConfig* cfg, bool force_global) {
+// Ndim <= SMALL_MAX_N without full-matrix outputs: warps without a workspace (the
+// CTA-wide kernel stays for full matrices and the forced global-memory inverse)
+static cudaError_t small_config(int N, DecimConfig* cfg) {
+  cfg->small = 1;
+  cfg->threads = 128;
+  cfg->smem = 0;
+  const void* fn = N <= 4 ? (const void*)k_decimate_small<4> : (const void*)k_decimate_small<8>;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cfg->ctas_per_sm, fn, cfg->threads, 0);
+}
+
+cudaError_t decim_fp64_config(int N, int threads_override, DecimConfig* cfg, bool force_global,
+                              bool full_out) {
+  if (N <= SMALL_MAX_N && !force_global && !full_out) return small_config(N, cfg);
   if (fp64_split(N)) {
     const cudaError_t e = split64_config(N, cfg);
     cfg->inv_global = force_global ? 1 : 0;       // of the FP64 fallback inverse
@@ -230,6 +288,11 @@ cudaError_t decim_fp64_config(int N, int threads_override, DecimConfig* cfg, boo
 cudaError_t launch_decimate_fp64(const DecimArgs& a, const DecimConfig& cfg, int grid,
                                  cudaStream_t s) {
   if (cfg.split) return launch_split64(a, cfg, grid, s);
+  if (cfg.small) {
+    if (a.N <= 4) k_decimate_small<4><<<grid, cfg.threads, 0, s>>>(a);
+    else k_decimate_small<8><<<grid, cfg.threads, 0, s>>>(a);
+    return cudaGetLastError();
+  }
   if (cfg.inv_global) {
     k_decimate_fp64<13, true><<<grid, cfg.threads, cfg.smem, s>>>(a);
     return cudaGetLastError();

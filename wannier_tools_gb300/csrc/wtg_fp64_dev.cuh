@@ -181,6 +181,16 @@ __device__ double cta_gemm_db(const double2* __restrict__ X, const double2* __re
   return nrm;
 }
 
+__device__ __forceinline__ float d2f_bits(double x) {    // truncating FP64 -> FP32
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  const uint32_t sign = (uint32_t)(u >> 63) << 31;
+  const int ex = (int)((u >> 52) & 0x7FF);
+  const int e32 = ex - 1023 + 127;
+  if (ex == 0 || e32 <= 0) return __uint_as_float(sign);
+  if (e32 >= 255) return __uint_as_float(sign | 0x7F800000u);
+  return __uint_as_float(sign | ((uint32_t)e32 << 23) | (uint32_t)((u >> 29) & 0x7FFFFFu));
+}
+
 constexpr int GJ_PANEL = 8;   // pivot steps per pass of the global-memory Gauss-Jordan
 
 struct Shared {
@@ -217,6 +227,13 @@ __device__ __forceinline__ Shared fp64_layout(unsigned char* smraw, int N, int K
   s.cols = s.perm + N;
   s.misc = s.cols + N;
   return s;
+}
+
+// 1 / v, with the products' rounding spelled out: every elimination (a CTA's, a
+// warp's, in shared or global memory) has the same pivot reciprocals bit for bit
+__device__ __forceinline__ double2 crecip(double2 v) {
+  const double inv_d = 1.0 / fma(v.x, v.x, __dmul_rn(v.y, v.y));
+  return make_double2(v.x * inv_d, -v.y * inv_d);
 }
 
 // |re| + |im| (LAPACK's dcabs1, the izamax criterion) as an order-preserving
@@ -269,8 +286,7 @@ __device__ int gj_core(double2* __restrict__ sM, int n, int ld, const Shared& s)
           s.misc[1] = 1;
         } else {
           const double2 pv = sM[p + k * ld];
-          const double inv_d = 1.0 / (pv.x * pv.x + pv.y * pv.y);
-          s.recip[0] = make_double2(pv.x * inv_d, -pv.y * inv_d);
+          s.recip[0] = crecip(pv);
         }
       }
     }
@@ -382,8 +398,7 @@ __device__ int schur_block_invert(const double2* __restrict__ X, double2 w, int 
         if (lane == 0) s.misc[1] = 1;
       } else {
         const double2 pv = sM[p + k * N];
-        const double inv_d = 1.0 / (pv.x * pv.x + pv.y * pv.y);
-        const double2 r = make_double2(pv.x * inv_d, -pv.y * inv_d);
+        const double2 r = crecip(pv);
         // multipliers of the rows below k after the swap k <-> p, and the pivot row
         for (int i = k + 1 + lane; i < N; i += 32)
           s.colbuf[i] = cmul(sM[(i == p ? k : i) + k * N], r);
@@ -485,8 +500,7 @@ __device__ int schur_block_invert_global(const double2* __restrict__ X, double2 
         if (lane == 0) s.misc[1] = 1;
       } else {
         const double2 pv = Mg[p + (size_t)k * N];
-        const double inv_d = 1.0 / (pv.x * pv.x + pv.y * pv.y);
-        const double2 r = make_double2(pv.x * inv_d, -pv.y * inv_d);
+        const double2 r = crecip(pv);
         for (int i = k + 1 + lane; i < N; i += 32)
           s.colbuf[i] = cmul(Mg[(i == p ? k : i) + (size_t)k * N], r);
         for (int j = k + 1 + lane; j < N; j += 32) s.rowbuf[j] = Mg[p + (size_t)j * N];
@@ -595,8 +609,7 @@ __device__ int gj_invert_global(const double2* __restrict__ X, double2 w, int N,
             s.misc[1] = 1;
           } else {
             const double2 pv = P[p + t * N];
-            const double inv_d = 1.0 / (pv.x * pv.x + pv.y * pv.y);
-            s.recip[t] = make_double2(pv.x * inv_d, -pv.y * inv_d);
+            s.recip[t] = crecip(pv);
           }
         }
       }

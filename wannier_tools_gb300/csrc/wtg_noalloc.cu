@@ -22,6 +22,7 @@
 //     rewritten per instance by the kernel), and calls whose kernels overlap on
 //     the GPU (different streams, or different host threads) race on it — the
 //     caller must order them.
+#include <climits>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -104,7 +105,7 @@ extern "C" int wtg_surfgreen_batch_noalloc(int ndim, int nw, int nk, const doubl
   e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return nerr(WTG_ECUDA, cudaGetErrorString(e));
   const long long n_inst = (long long)nk * nomega;
-  const size_t fit = (WTG_NOALLOC_SCRATCH_BYTES - counter_bytes) / per_cta;
+  const size_t fit = per_cta ? (WTG_NOALLOC_SCRATCH_BYTES - counter_bytes) / per_cta : INT_MAX;
   long long grid = (long long)cfg.ctas_per_sm * nsm;
   if ((long long)fit < grid) grid = (long long)fit;
   // every CTA takes one more ticket from the counter after the last instance, so the

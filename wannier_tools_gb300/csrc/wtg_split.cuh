@@ -189,16 +189,6 @@ __device__ __forceinline__ double assemble_fast(long long S, int be0) {
   return __hiloint2double((int)(a != 0 ? hi : 0u), (int)(a != 0 ? (unsigned)m : 0u));
 }
 
-__device__ __forceinline__ float d2f_bits(double x) {    // truncating FP64 -> FP32
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const uint32_t sign = (uint32_t)(u >> 63) << 31;
-  const int ex = (int)((u >> 52) & 0x7FF);
-  const int e32 = ex - 1023 + 127;
-  if (ex == 0 || e32 <= 0) return __uint_as_float(sign);
-  if (e32 >= 255) return __uint_as_float(sign | 0x7F800000u);
-  return __uint_as_float(sign | ((uint32_t)e32 << 23) | (uint32_t)((u >> 29) & 0x7FFFFFu));
-}
-
 __device__ __forceinline__ double f2d_bits(float f) {     // exact FP32 -> FP64
   const uint32_t w = __float_as_uint(f);
   const unsigned long long sign = (unsigned long long)(w >> 31) << 63;

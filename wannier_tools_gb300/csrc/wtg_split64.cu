@@ -34,6 +34,7 @@ namespace {
 #include "wtg_split.cuh"
 #include "wtg_split_inverse.cuh"
 #include "wtg_fp64_solve.cuh"
+#include "wtg_small_dev.cuh"
 
 // Decimation of one instance whose eps, eps_s, eps_t (= H00), alpha (= H01) and
 // beta (= H01^dagger) already sit in workspace matrices 0..4 of W (11 N x N
@@ -200,7 +201,10 @@ __global__ void __launch_bounds__(SP_T, 1) k_batch_split64(const __grid_constant
       if (a.status) a.status[p] = (uint8_t)st;
     };
     constexpr int KC = 16;
-    if (m.N > FP64_SPLIT_MAX_N) {
+    if (m.N <= SMALL_MAX_N) {                // one warp, as k_decimate_small
+      if (tid < 32) small_point(m.N, w, o, W, emit);
+      __syncthreads();
+    } else if (m.N > FP64_SPLIT_MAX_N) {
       fp64_solve<13, true>(m.N, KC, w, o, nullptr, nullptr, nullptr, W,
                            fp64_layout(smem_dyn, m.N, KC, false), emit);
     } else if (m.N < FP64_SPLIT_MIN_N) {
