@@ -69,6 +69,16 @@ def test_nonfinite_hamiltonian_is_flagged(built_lib):
         assert (r["iters"] == 5).all()
 
 
+# columns of NaN alone: no row is a pivot candidate, at instance numbers above Ndim too
+@pytest.mark.parametrize("nw,np_,nk", [(2, 2, 300), (8, 2, 300), (20, 2, 200), (56, 2, 160), (88, 3, 3)])
+def test_nonfinite_instances(built_lib, nw, np_, nk):
+    m = synthetic.make_model(nw, np_, seed=6)
+    h = np.full_like(m.hmnr, np.nan)
+    with api.Model(h, m.irvec, m.ndegen, np_) as g:
+        r = g.surface_spectrum(np.zeros((nk, 2)), [0.0], 1e-2 * EV, [1], [1], itermax=2)
+    assert (r["status"] & PT_NONFINITE).all() and (r["status"] & PT_NOT_CONVERGED).all()
+
+
 @pytest.mark.parametrize("nw,np_", [(12, 2), (5, 5), (32, 2), (65, 1), (43, 3), (54, 3), (97, 2)])
 def test_spectra_vs_oracle(built_lib, nw, np_):
     m = synthetic.make_model(nw, np_, seed=nw)

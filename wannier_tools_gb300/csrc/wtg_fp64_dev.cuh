@@ -277,7 +277,7 @@ __device__ int gj_core(double2* __restrict__ sM, int n, int ld, const Shared& s)
           bi = oi;
         }
       }
-      const int p = bi;
+      const int p = best < 0 ? k : bi;     // a column of NaN alone has no candidate
       // column k after the row swap k <-> p (entry k itself is not used)
       for (int i = lane; i < n; i += 32) s.colbuf[i] = sM[(i == p ? k : i) + k * ld];
       if (lane == 0) {
@@ -393,7 +393,7 @@ __device__ int schur_block_invert(const double2* __restrict__ X, double2 w, int 
           bi = oi;
         }
       }
-      const int p = bi;
+      const int p = best < 0 ? k : bi;     // a column of NaN alone has no candidate
       if (best == 0) {
         if (lane == 0) s.misc[1] = 1;
       } else {
@@ -495,7 +495,7 @@ __device__ int schur_block_invert_global(const double2* __restrict__ X, double2 
           bi = oi;
         }
       }
-      const int p = bi;
+      const int p = best < 0 ? k : bi;     // a column of NaN alone has no candidate
       if (best == 0) {
         if (lane == 0) s.misc[1] = 1;
       } else {
@@ -601,7 +601,7 @@ __device__ int gj_invert_global(const double2* __restrict__ X, double2 w, int N,
             bi = oi;
           }
         }
-        const int p = bi;
+        const int p = best < 0 ? k : bi;     // a column of NaN alone has no candidate
         for (int i = lane; i < N; i += 32) Cm[i + t * N] = P[(i == p ? k : i) + t * N];
         if (lane == 0) {
           s.perm[k] = p;

@@ -1148,7 +1148,7 @@ __device__ __forceinline__ void gj_pivot_publish(const unsigned long long (&x)[R
 #pragma unroll
   for (int m = 0; m < R; ++m) ps[m] = pos_of[min(lane + 32 * m, N - 1)];
   unsigned bkey = 0;                      // key + 1; 0: no candidate
-  int bpos = 0x7fffffff, bm = 0;
+  int bpos = t, bm = 0;                   // (a valid position where a key wraps to none)
   float2 bv = make_float2(0.f, 0.f);
 #pragma unroll
   for (int m = 0; m < R; ++m) {
