@@ -49,6 +49,7 @@ constexpr int PT_TIMEOUT = 8;
 constexpr int MX_MAXN = 320;           // largest Ndim
 constexpr int MX_SMEM_GJ_N = 112;      // up to here the FP32 Gauss-Jordan runs in shared memory
 constexpr int MX_PANEL = 16;           // pivot steps per panel of the global-memory Gauss-Jordan
+constexpr int GJS_PANEL = 8;           // and of the shared-memory one
 constexpr int MX_ROWS = MX_MAXN / 32;  // rows per lane of a register-resident column
 constexpr int EXP_MIN = 80;            // shared exponents are at least this (biased): rows and
                                        // columns below 2^-940 count as zero
@@ -516,6 +517,7 @@ struct SplitTail {
   int misc[5];                   // 0 instance, 1 singular, 2-3 pivot rows (shared-memory Gauss-Jordan)
 };
 constexpr int SPLIT_TAIL = (int)sizeof(SplitTail);
+static_assert(2 * GJS_PANEL <= MX_PANEL, "two panels' multipliers and reciprocals");
 // the FP32 Gauss-Jordan areas (matrix and multipliers) fit below the exponents for
 // every stage width
 static_assert((MX_SMEM_GJ_N + MX_PANEL) * MX_SMEM_GJ_N * 8 <= 2 * 2 * MAXD * APLANE, "FP32 GJ area");
@@ -1140,7 +1142,7 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 // division and no shuffle.
 template <int R>
 __device__ __forceinline__ void gj_pivot_publish(const unsigned long long (&x)[R], int t, int N,
-                                                 float2* cb, float2* rslot, int* prow, int* misc,
+                                                 float2* cb, float2* rslot, int* prow, int* singular,
                                                  int* pos_of, int* row_at) {
   const int lane = threadIdx.x & 31;
   const int rk = row_at[t];              // moves to the pivot's position
@@ -1176,7 +1178,7 @@ __device__ __forceinline__ void gj_pivot_publish(const unsigned long long (&x)[R
     pos_of[rk] = bpos;
     row_at[t] = brow;
     pos_of[brow] = t;
-    if (kmax == 1u) misc[1] = 1;
+    if (kmax == 1u) *singular = 1;
     else *rslot = rc;
   }
 }
@@ -1237,25 +1239,32 @@ __device__ __forceinline__ void gj_step_cols(unsigned long long (&x)[C][R],
 #undef WTG_GJ_AT
 }
 
+// barrier of the panel's warps (0 .. GJS_PANEL-1)
+__device__ __forceinline__ void gj_panel_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(32 * GJS_PANEL) : "memory");
+}
+
 // M = w I - X (FP64, kept in Mi for the refinement, with its row exponents),
 // then FP32 Gauss-Jordan with partial pivoting into G (FP64, with its row and
 // column exponents).  Returns 1 on an exact zero pivot (G = identity then).
 // Ndim <= 112, the matrix in shared memory.  The pivot steps run in panels of
-// MX_PANEL columns: a panel's columns stay in registers, one per warp (lane l
-// holds rows l, l + 32, ...); each step updates them with one barrier, the owner
-// of the next column finding the next pivot and publishing its multiplier
-// column (look-ahead).  Then every other column is read once into registers, up
-// to six per warp, put through the panel's steps and written back.  Rows stay in
-// place (gj_pivot_publish); the output reads them back in pivot order.
-// At Ndim 112 an inverse takes 374 k cycles, half of it the 112 pivot steps'
-// latency; a step-by-step form (every column through shared memory each step,
-// 4-way selects instead of a branch on the pivot's row slot) took 597 k.  Same
-// operations per entry, in the same order.
+// GJS_PANEL columns, one panel ahead of the rest: warps 0 .. GJS_PANEL-1 hold the
+// next panel's columns in registers (lane l holds rows l, l + 32, ...), put them
+// through the current panel's steps and factor them, one named barrier a step, the
+// owner of the next column finding the next pivot and publishing its multiplier
+// column; meanwhile the other warps read every remaining column once, up to C at a
+// time, and put it through the current panel's steps.  Rows stay in place
+// (gj_pivot_publish); the output reads them back in pivot order.
+// What bounds it: the latency of the pivot steps (search, publication, barrier;
+// about 1.4 k cycles each).  Alone on the chip an inverse takes 147.8 us at Ndim
+// 112 and 32.9 at 40; with panels of 16 by all warps and the rest after each panel
+// 172.5 and 37.9; panels of 4 175.2 and 35.1; panels factored by one warp in
+// registers 232 and 37.0.  Same operations per entry, in the same order, in all.
 template <int R>
 __device__ __noinline__ int gj32_start(const double2* __restrict__ X, double2 w, int N,
                                        double2* __restrict__ const W, int iM, int iG,
                                        const MxShared s) {
-  constexpr int C = R == 2 ? 3 : 6;       // 16 warps x C columns >= 32 R - MX_PANEL
+  constexpr int C = R == 2 ? 3 : 6;       // trailing columns a warp holds at a time
   const size_t NN = (size_t)N * N;
   double2* __restrict__ const Mi = W + iM * NN;
   double2* __restrict__ const G = W + iG * NN;
@@ -1263,9 +1272,9 @@ __device__ __noinline__ int gj32_start(const double2* __restrict__ X, double2 w,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int nwarp = SP_T / 32;
   float2* __restrict__ sM = reinterpret_cast<float2*>(s.base());
-  float2* __restrict__ Cm = sM + (size_t)N * N;          // [MX_PANEL][N] multiplier columns
-  float2* __restrict__ recip = sh.recip;
-  int* __restrict__ prow = sh.prow;                      // pivot rows of the panel's steps
+  float2* __restrict__ Cm = sM + (size_t)N * N;          // [2][GJS_PANEL][N] multiplier columns
+  float2* __restrict__ recip = sh.recip;                 // [2][GJS_PANEL]
+  int* __restrict__ prow = sh.prow;                      // pivot rows
   int* __restrict__ misc = sh.misc;
   int* __restrict__ pos_of = sh.pos_of;
   int* __restrict__ row_at = sh.row_at;
@@ -1297,72 +1306,89 @@ __device__ __noinline__ int gj32_start(const double2* __restrict__ X, double2 w,
     eM[i] = EXP_MIN;
     eGr[i] = EXP_MIN;
   }
-  if (tid == 0) misc[1] = 0;
+  if (tid < 2) misc[2 + tid] = 0;
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < R; ++q)
     if (lane + 32 * q < N) atomicMax(&eM[lane + 32 * q], rmax[q]);
-  for (int k0 = 0; k0 < N; k0 += MX_PANEL) {
-    const int pb = min(MX_PANEL, N - k0);
-    unsigned long long xp[1][R];          // this warp's panel column
+  // warps 0 .. GJS_PANEL-1, a column each: the panel at k0 (pb columns) through the
+  // pbb steps of the panel before it, factored into buffer b, and written back
+  auto panel = [&](int k0, int pb, int pbb, int b) {
+    float2* const cm = Cm + b * GJS_PANEL * N;
+    const float2* const cb = Cm + (b ^ 1) * GJS_PANEL * N;
+    float2* const rc = recip + b * GJS_PANEL;
+    float2* const col = sM + (size_t)(k0 + warp) * N;
+    unsigned long long xp[1][R];
 #pragma unroll
     for (int m = 0; m < R; ++m) {
       const int i = lane + 32 * m;
-      const float2 v = (warp < pb && i < N) ? sM[(size_t)(k0 + warp) * N + i] : make_float2(0.f, 0.f);
+      const float2 v = (warp < pb && i < N) ? col[i] : make_float2(0.f, 0.f);
       xp[0][m] = pack2(v.x, v.y);
     }
+    if (warp < pb)
+      for (int t = 0; t < pbb; ++t)
+        gj_step_cols<R, 1>(xp, cb + t * N, N, prow[k0 - pbb + t], recip[(b ^ 1) * GJS_PANEL + t], -1);
     auto publish = [&](int t) {
-      gj_pivot_publish<R>(xp[0], k0 + t, N, Cm + t * N, &recip[t], prow, misc, pos_of, row_at);
+      gj_pivot_publish<R>(xp[0], k0 + t, N, cm + t * N, rc + t, prow, misc + 2 + b, pos_of, row_at);
     };
     if (warp == 0) publish(0);
-    __syncthreads();
+    gj_panel_sync();
     for (int t = 0; t < pb; ++t) {
-      if (misc[1]) break;
+      if (misc[2 + b]) break;
       if (warp < pb) {
-        gj_step_cols<R, 1>(xp, Cm + t * N, N, prow[k0 + t], recip[t], warp == t ? 0 : -1);
+        gj_step_cols<R, 1>(xp, cm + t * N, N, prow[k0 + t], rc[t], warp == t ? 0 : -1);
         if (warp == t + 1) publish(t + 1);
       }
-      __syncthreads();
+      gj_panel_sync();
     }
-    if (misc[1]) break;
-    if (warp < pb) {                      // panel column back to shared memory
+    if (warp < pb) {
 #pragma unroll
       for (int m = 0; m < R; ++m) {
         const int i = lane + 32 * m;
-        if (i < N) sM[(size_t)(k0 + warp) * N + i] = unpack2(xp[0][m]);
+        if (i < N) col[i] = unpack2(xp[0][m]);
       }
     }
-    // this warp's other columns through the panel's steps
-    const int nt = N - pb, nc = warp < nt ? (nt - warp + nwarp - 1) / nwarp : 0;
-    if (nc > 0) {
-      unsigned long long x[C][R];
+  };
+  if (warp < GJS_PANEL) panel(0, min(GJS_PANEL, N), 0, 0);
+  __syncthreads();
+  for (int k0 = 0, b = 0; k0 < N && !misc[2 + b]; k0 += GJS_PANEL, b ^= 1) {
+    const int pb = min(GJS_PANEL, N - k0), pn = min(GJS_PANEL, N - k0 - pb);
+    if (pn > 0 && warp < GJS_PANEL) {
+      panel(k0 + pb, pn, pb, b ^ 1);
+    } else {
+      // the columns outside the two panels (after the last one every warp's), C at a time
+      const int first = pn > 0 ? GJS_PANEL : 0, step = nwarp - first, skip = pb + pn;
+      const float2* const cm = Cm + b * GJS_PANEL * N;
+      for (int o0 = warp - first; o0 < N - skip; o0 += C * step) {
+        unsigned long long x[C][R];
 #pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const int o = warp + c * nwarp;
-        const float2* col = sM + (size_t)(o < k0 ? o : o + pb) * N;
+        for (int c = 0; c < C; ++c) {
+          const int o = o0 + c * step;
+          const float2* col = sM + (size_t)(o < k0 ? o : o + skip) * N;
 #pragma unroll
-        for (int m = 0; m < R; ++m) {
-          const int i = lane + 32 * m;
-          const float2 v = (c < nc && i < N) ? col[i] : make_float2(0.f, 0.f);
-          x[c][m] = pack2(v.x, v.y);
+          for (int m = 0; m < R; ++m) {
+            const int i = lane + 32 * m;
+            const float2 v = (o < N - skip && i < N) ? col[i] : make_float2(0.f, 0.f);
+            x[c][m] = pack2(v.x, v.y);
+          }
         }
-      }
-      for (int t = 0; t < pb; ++t)
-        gj_step_cols<R, C>(x, Cm + t * N, N, prow[k0 + t], recip[t], -1);
+        for (int t = 0; t < pb; ++t)
+          gj_step_cols<R, C>(x, cm + t * N, N, prow[k0 + t], recip[b * GJS_PANEL + t], -1);
 #pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const int o = warp + c * nwarp;
-        float2* col = sM + (size_t)(o < k0 ? o : o + pb) * N;
+        for (int c = 0; c < C; ++c) {
+          const int o = o0 + c * step;
+          float2* col = sM + (size_t)(o < k0 ? o : o + skip) * N;
 #pragma unroll
-        for (int m = 0; m < R; ++m) {
-          const int i = lane + 32 * m;
-          if (c < nc && i < N) col[i] = unpack2(x[c][m]);
+          for (int m = 0; m < R; ++m) {
+            const int i = lane + 32 * m;
+            if (o < N - skip && i < N) col[i] = unpack2(x[c][m]);
+          }
         }
       }
     }
     __syncthreads();
   }
-  const int singular = misc[1];
+  const int singular = misc[2] | misc[3];
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < R; ++q) rmax[q] = 0;
@@ -1466,7 +1492,7 @@ __device__ __noinline__ int gj32_global(const double2* __restrict__ X, double2 w
         xp[0][m] = pack2(v.x, v.y);
       }
       auto publish = [&](int t) {
-        gj_pivot_publish<R>(xp[0], k0 + t, N, Cm + t * N, &recip[t], prow, misc, pos_of, row_at);
+        gj_pivot_publish<R>(xp[0], k0 + t, N, Cm + t * N, &recip[t], prow, misc + 1, pos_of, row_at);
       };
       if (warp == 0) publish(0);
       __syncthreads();
