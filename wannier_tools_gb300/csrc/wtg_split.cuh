@@ -171,6 +171,11 @@ __device__ __forceinline__ double assemble(long long S, int be0) {
   return __longlong_as_double((long long)(r | ((unsigned long long)sg << 63)));
 }
 
+// a b + c, one instruction of the multiply pipe
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+  return (long long)a * b + c;
+}
+
 // assemble for |S| < 2^63, with the common case (zero, or |S| >= 2^32 and a normal
 // result) in about half the instructions: the drain of the accumulators is
 // bound by the integer pipe
@@ -178,16 +183,17 @@ template <bool ROUND>
 __device__ __forceinline__ double assemble_fast(long long S, int be0) {
   const long long sg = S >> 63;
   const unsigned long long a = (unsigned long long)((S ^ sg) - sg);
-  const unsigned ah = (unsigned)(a >> 32);
-  const int lz = __clz((int)ah);
-  const int be = 63 - lz + be0;
-  if (a != 0 && (ah == 0 || (unsigned)(be - 1) >= 2045u)) return assemble<ROUND>(S, be0);
-  unsigned long long n = a << ((lz - 1) & 63);        // leading bit at 62
+  const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a;
+  const int lz = __clz((int)ah);                      // 1..31, or 32 (zero, or below 2^32)
+  const unsigned be1 = (unsigned)(62 - lz + be0);
+  if (ah == 0 ? al != 0 : be1 >= 2045u) return assemble<ROUND>(S, be0);
+  // leading bit at 62: two 32-bit shifts
+  unsigned long long n =
+      ((unsigned long long)__funnelshift_l(al, ah, (unsigned)lz - 1) << 32) | (al << ((lz - 1) & 31));
   if (ROUND) n += 0x200;
   const unsigned long long m = n >> 10;               // the hidden bit adds 1 to the exponent
-  const unsigned hi = ((unsigned)(m >> 32) + ((unsigned)(be - 1) << 20)) |
-                      ((unsigned)(sg >> 32) & 0x80000000u);
-  return __hiloint2double((int)(a != 0 ? hi : 0u), (int)(a != 0 ? (unsigned)m : 0u));
+  const unsigned hi = ((unsigned)(m >> 32) + (be1 << 20)) | ((unsigned)(S >> 32) & 0x80000000u);
+  return __hiloint2double((int)(ah ? hi : 0u), (int)(unsigned)m);
 }
 
 __device__ __forceinline__ double f2d_bits(float f) {     // exact FP32 -> FP64
@@ -409,14 +415,14 @@ struct DigF8 {
                               fmaf(__uint_as_float(v[6]), 0x1p-6f, 4.0f * __uint_as_float(v[5])));
       const int low = __float2int_rn(f789);
       const int m2 = __float_as_int(__uint_as_float(v[0]) + 12582912.0f);      // + 0x4B400000
-      const long long S = ((long long)f2i(v[2]) * (1ll << 26) + (long long)f2i(v[3]) * (1ll << 18)) +
-                          ((long long)f2i(v[4]) * (1ll << 10) + (long long)low);
+      const long long S = mad_wide(f2i(v[2]), 1 << 26,
+                                   mad_wide(f2i(v[3]), 1 << 18, mad_wide(f2i(v[4]), 1 << 10, low)));
       const unsigned top = (unsigned)m2 * 1024u + ((unsigned)f2i(v[1]) * 4u);  // in units of 2^32
       return assemble_fast<true>(S + (long long)((unsigned long long)top << 32),
                                  ee - 2152 + 54 + 1023);
     } else {
-      const long long S = ((long long)f2i(v[0]) * (1ll << 24) + (long long)f2i(v[1]) * (1ll << 16)) +
-                          ((long long)f2i(v[2]) * (1ll << 8) + (long long)f2i(v[3]));
+      const long long S = mad_wide(f2i(v[0]), 1 << 24,
+                                   mad_wide(f2i(v[1]), 1 << 16, mad_wide(f2i(v[2]), 1 << 8, f2i(v[3]))));
       return assemble_fast<true>(S, ee - 2152 + 72 + 1023);
     }
   }
@@ -830,6 +836,21 @@ __device__ __noinline__ int split_generate(const double2* __restrict__ W, uint32
   return 0;
 }
 
+// a - b where it stands: not computed ahead of the branch around it (two FP64
+// operations a clock: speculated subtractions cost a tenth of a product)
+__device__ __forceinline__ double dsub_here(double a, double b) {
+  double r;
+  asm volatile("sub.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+}
+
+// |x| from its upper word: the magnitude truncated to 21 bits, 0 or Inf outside
+// FP32's range (the sums it goes into are compared with margins far above 2^-20)
+__device__ __forceinline__ float upper_f32(double x) {
+  const int h = (__double2hiint(x) & 0x7FFFFFFF) - (896 << 20);
+  return __int_as_float(min(max(h, 0), 0x0FF00000) << 3);
+}
+
 // Accumulators of a tile through the epilogue (all warps: four per quadrant of
 // 32 tensor-memory lanes, each taking 4 of every 16 columns).  Returns this
 // thread's part of the product's FP32 sum.
@@ -925,9 +946,10 @@ __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, 
           if (first) {
             val[jj] = make_double2(-val[jj].x, -val[jj].y);
             // (one of the warp's rows is on the diagonal; FP64 adds are not free: two a clock)
-            if ((unsigned)(j0 + jj - rb0 - quad * 32) < 32u && rowL == j0 + jj) val[jj].x += 1.0;
+            if ((unsigned)(j0 + jj - rb0 - quad * 32) < 32u && rowL == j0 + jj)
+              val[jj].x = dsub_here(val[jj].x, -1.0);
           } else {
-            val[jj] = make_double2(old0[jj].x - val[jj].x, old0[jj].y - val[jj].y);
+            val[jj] = make_double2(dsub_here(old0[jj].x, val[jj].x), dsub_here(old0[jj].y, val[jj].y));
           }
         }
       } else if (epi == OZ_ADDTO || !first) {
@@ -944,9 +966,9 @@ __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, 
 #pragma unroll
         for (int jj = 0; jj < 2; ++jj) {
           if (!(jj ? on1 : on0)) continue;
-          const float fr = d2f_bits(val[jj].x), fi = d2f_bits(val[jj].y);
+          const float fr = upper_f32(val[jj].x), fi = upper_f32(val[jj].y);
           if (K::FRO && epi == OZ_IMINUS) nrm = fmaf(fr, fr, fmaf(fi, fi, nrm));
-          else nrm += fabsf(fr) + fabsf(fi);
+          else nrm += fr + fi;
         }
       }
       unsigned e[2];
