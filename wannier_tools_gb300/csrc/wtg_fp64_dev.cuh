@@ -260,7 +260,7 @@ __device__ int gj_core(double2* __restrict__ sM, int n, int ld, const Shared& s)
   for (int k = 0; k < n; ++k) {
     if (warp == 0) {
       long long best = -1;
-      int bi = n;
+      int bi = k;                 // where no row is a candidate (NaN alone)
       for (int i = k + lane; i < n; i += 32) {
         const long long v = cabs1_key(sM[i + k * ld]);
         if (v > best) {
@@ -277,7 +277,7 @@ __device__ int gj_core(double2* __restrict__ sM, int n, int ld, const Shared& s)
           bi = oi;
         }
       }
-      const int p = best < 0 ? k : bi;     // a column of NaN alone has no candidate
+      const int p = bi;
       // column k after the row swap k <-> p (entry k itself is not used)
       for (int i = lane; i < n; i += 32) s.colbuf[i] = sM[(i == p ? k : i) + k * ld];
       if (lane == 0) {
@@ -376,7 +376,7 @@ __device__ int schur_block_invert(const double2* __restrict__ X, double2 w, int 
   for (int k = 0; k < m; ++k) {
     if (warp == 0) {
       long long best = -1;
-      int bi = m;
+      int bi = k;                 // where no row is a candidate (NaN alone)
       for (int i = k + lane; i < m; i += 32) {
         const long long v = cabs1_key(sM[i + k * N]);
         if (v > best) {
@@ -393,7 +393,7 @@ __device__ int schur_block_invert(const double2* __restrict__ X, double2 w, int 
           bi = oi;
         }
       }
-      const int p = best < 0 ? k : bi;     // a column of NaN alone has no candidate
+      const int p = bi;
       if (best == 0) {
         if (lane == 0) s.misc[1] = 1;
       } else {
@@ -478,7 +478,7 @@ __device__ int schur_block_invert_global(const double2* __restrict__ X, double2 
   for (int k = 0; k < m; ++k) {
     if (warp == 0) {
       long long best = -1;
-      int bi = m;
+      int bi = k;                 // where no row is a candidate (NaN alone)
       for (int i = k + lane; i < m; i += 32) {
         const long long v = cabs1_key(Mg[i + (size_t)k * N]);
         if (v > best) {
@@ -495,7 +495,7 @@ __device__ int schur_block_invert_global(const double2* __restrict__ X, double2 
           bi = oi;
         }
       }
-      const int p = best < 0 ? k : bi;     // a column of NaN alone has no candidate
+      const int p = bi;
       if (best == 0) {
         if (lane == 0) s.misc[1] = 1;
       } else {
@@ -584,7 +584,7 @@ __device__ int gj_invert_global(const double2* __restrict__ X, double2 w, int N,
       const int k = k0 + t;
       if (warp == 0) {
         long long best = -1;
-        int bi = N;
+        int bi = k;                 // where no row is a candidate (NaN alone)
         for (int i = k + lane; i < N; i += 32) {
           const long long v = cabs1_key(P[i + t * N]);
           if (v > best) {
@@ -601,7 +601,7 @@ __device__ int gj_invert_global(const double2* __restrict__ X, double2 w, int N,
             bi = oi;
           }
         }
-        const int p = best < 0 ? k : bi;     // a column of NaN alone has no candidate
+        const int p = bi;
         for (int i = lane; i < N; i += 32) Cm[i + t * N] = P[(i == p ? k : i) + t * N];
         if (lane == 0) {
           s.perm[k] = p;
