@@ -406,9 +406,36 @@ class SpectrumRun:
         iteration count of each point (both forms iterate alike within +-1)."""
         import numpy as np
         prof, its = r["prof"], r["its"]
+        m = self.m
         launch_ms = prof["decim_ms"] / max(1, prof["decim_launches"])
         alg = float(((56.0 * its + 24.0) * self.n3).sum())
         ach = alg / (prof["decim_ms"] / 1e3) / 1e12 if prof["decim_ms"] > 0 else None
+        npad = (m.ndim + 7) // 8 * 8
+        nch = (m.ndim + 15) // 16
+        nrb = (m.ndim + 127) // 128
+        # MMA flops of one slice pair of a complex product: row blocks of 128 x 2 components x
+        # K chunks x 2 real products x 2*128*16 flops per output column over Ndim columns
+        # rounded up to 8
+        pair = nrb * 2 * nch * 2 * 2.0 * 128 * 16 * npad
+        fp64_best = max(peaks["dfma"], peaks["dmma"])
+        if f == "fp64" and 25 <= m.ndim <= 256:
+            # exactly split products: per iteration six loop products and two residuals of 34
+            # slice pairs, two corrections of 10
+            issued = float(((8 * 34 + 2 * 10) * its * pair).sum())
+            iss = issued / (prof["decim_ms"] / 1e3) / 1e12 if prof["decim_ms"] > 0 else None
+            peak = MEASURED_PEAKS.get("bf16_tflops")
+            traffic = traffic_per_solve(self.wl_name(), "k_decimate_split64")
+            return {"bound": "tensor", "kernel": "k_decimate_split64", "achieved": ach, "peak": peak,
+                    "unit": "TFLOP/s", "frac": (ach / peak) if (ach and peak) else None,
+                    "traffic": (traffic * self.B * self.nomega) if traffic else None,
+                    "traffic_unit": "bytes per launch",
+                    "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst; F16 MMAs run at its rate)",
+                    "launch_ms": launch_ms, "dfma_peak": peaks["dfma"], "dmma_peak": peaks["dmma"],
+                    "work": "(56*it+24)*Ndim^3 FP64 flops per solve (algorithmic), it = FP64 iterations",
+                    "issued_f16_tflops": iss, "issued_frac": (iss / peak) if (iss and peak) else None,
+                    "issued_work": "F16 MMA flops issued in the loop: per iteration 8 products of 34 "
+                                   "slice pairs and 2 of 10",
+                    "vs_fp64_peak": (ach / fp64_best) if ach else None}
         if f == "fp64":
             peak = max(peaks["dfma"], peaks["dmma"])
             traffic = traffic_per_solve(self.wl_name())
@@ -422,16 +449,9 @@ class SpectrumRun:
                                    "wtg_probe_dmma_peak)",
                     "dfma_peak": peaks["dfma"], "dmma_peak": peaks["dmma"], "launch_ms": launch_ms,
                     "work": "(56*it+24)*Ndim^3 flops per solve, it = FP64 iterations"}
-        m = self.m
-        npad = (m.ndim + 7) // 8 * 8
-        nch = (m.ndim + 15) // 16
-        nrb = (m.ndim + 127) // 128
-        # BF16 MMA flops issued by one 7-digit complex product: row blocks of 128 x 2
-        # components x K chunks x 28 slice pairs x 2 real products x 2*128*16 flops per
-        # output column over Ndim columns rounded up to 8; 7 such products per iteration (six loop products
-        # and the refinement's residual), the 4-digit correction (10 pairs) as 10/28 of one
-        per_prod = nrb * 2 * nch * 56 * 2.0 * 128 * 16 * npad
-        issued = float(((7.0 + 10.0 / 28.0) * its * per_prod).sum())
+        # BF16 MMA flops issued in the loop: 7 products of 28 slice pairs per iteration (six
+        # loop products and the refinement's residual), the 4-digit correction of 10
+        issued = float(((7 * 28 + 10) * its * pair).sum())
         iss = issued / (prof["decim_ms"] / 1e3) / 1e12 if prof["decim_ms"] > 0 else None
         peak = MEASURED_PEAKS.get("bf16_tflops")
         return {"bound": "tensor", "kernel": "k_decimate_mixed", "achieved": ach, "peak": peak,
@@ -442,7 +462,7 @@ class SpectrumRun:
                 "issued_work": "BF16 MMA flops issued: per iteration 7 products of 28 slice pairs and "
                                "one of 10, each ceil(Ndim/128) row blocks x 2 components x "
                                "ceil(Ndim/16) K chunks x 2*128*16 flops per column x Ndim columns rounded up to 8",
-                "vs_fp64_peak": (ach / max(peaks["dfma"], peaks["dmma"])) if ach else None}
+                "vs_fp64_peak": (ach / fp64_best) if ach else None}
 
     def wl_name(self):
         for k, v in WORKLOADS.items():
@@ -876,10 +896,10 @@ def run_serve(args):
 
 # --- reference arm ---------------------------------------------------------------
 
-def traffic_per_solve(workload: str):
+def traffic_per_solve(workload: str, kernel: str = "k_decimate_fp64"):
     """DRAM bytes per solve of the decimation kernel from the committed ncu
-    summary (profiles/k_decimate_fp64_<workload>.md, line 'traffic_bytes_per_solve:')."""
-    p = ROOT / "profiles" / f"k_decimate_fp64_{workload}.md"
+    summary (profiles/<kernel>_<workload>.md, line 'traffic_bytes_per_solve:')."""
+    p = ROOT / "profiles" / f"{kernel}_{workload}.md"
     if not p.exists():
         return None
     for line in p.read_text().splitlines():

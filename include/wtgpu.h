@@ -53,11 +53,12 @@ extern "C" {
 #define WTG_PT_SINGULAR      2  /* exact zero pivot; the inverse is replaced by the
                                    identity, as zgesv+inv do (src/inverse.f90:51-55) */
 #define WTG_PT_NONFINITE     4  /* a spectral sum is NaN or Inf */
-#define WTG_PT_TIMEOUT       8  /* a bounded wait on the tensor cores gave up (mixed form);
-                                   the point's outputs are not valid */
+#define WTG_PT_TIMEOUT       8  /* a bounded wait on the tensor cores gave up (mixed form, and
+                                   the FP64 form at Ndim 25..256); the point's outputs are not
+                                   valid */
 
 /* precision modes */
-#define WTG_PREC_FP64  0        /* FP64 decimation; Ndim <= 320.  At Ndim 33..256 every product is
+#define WTG_PREC_FP64  0        /* FP64 decimation; Ndim <= 320.  At Ndim 25..256 every product is
                                    an exactly split product on the tcgen05 tensor cores (55-bit
                                    operands in balanced 8-bit digits, exact integer accumulation,
                                    smaller error than an FP64 product) and an inverse an FP32
@@ -349,8 +350,9 @@ int wtg_engine_graph_info(wtg_engine_t engine, int* graphs, long long* graph_lau
 /*
  * Tile table (the autotuner's output, wannier_tools_gb300/autotune.py): the
  * launch shape the kernels use at a given Ndim.
- *   WTG_PREC_FP64   value = threads per CTA of the per-model FP64 kernel, 128, 256
- *                   or 512 (Ndim above the shared-memory inverse always uses 256)
+ *   WTG_PREC_FP64   value = threads per CTA of the per-model kernel on the FP64 pipe,
+ *                   128, 256 or 512 (no effect at Ndim <= 8 and 25..256, which other
+ *                   kernels take, nor above, where it is always 256)
  *   WTG_PREC_MIXED  value = output-column pass width of the split-BF16 products, a
  *                   multiple of 8 up to 40
  * value 0 restores the built-in choice.  Results do not depend on the tile beyond

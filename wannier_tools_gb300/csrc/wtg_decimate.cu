@@ -14,8 +14,12 @@
 // followed by the spectral sums of src/surfstat.f90:149-160 /
 // src/fermiarc.f90:237-248.
 //
+// This file: the kernels on the FP64 pipe (Ndim <= 8 a few lanes of a warp per
+// instance, up to 24 and above 256 a CTA) and the routing; Ndim 25..256 runs on
+// exactly split tensor-core products (wtg_split64.cu).
+//
 // GB300 notes.  FP64 runs at 2 DFMA/clk/SM on this part (1.2 TFLOP/s measured,
-// with FP64 mma.sync slower still), so the kernel is bound by the FP64 pipe,
+// with FP64 mma.sync slower still), so the CTA kernel is bound by the FP64 pipe,
 // not by memory: the eight N x N matrices of an instance live in a per-CTA
 // global workspace (L2-resident), GEMM operands are staged through shared
 // memory in k-chunks, and the inverse runs in shared memory.  What matters is

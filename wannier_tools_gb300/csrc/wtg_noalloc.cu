@@ -6,9 +6,9 @@
 // fragments the pool), and latency-critical loops in which cudaMalloc /
 // cudaFree would synchronise the whole device and stall work on other
 // streams.  For them, wtg_surfgreen_batch_noalloc runs the FP64 decimation
-// kernel with its scratch (the per-CTA workspace of Ndim x Ndim complex
-// matrices, eleven or eight by Ndim, and the work counter) taken from the fixed array below instead of
-// from device allocations.  The caller passes every input and output as device
+// kernel with its scratch (the work counter and the per-CTA workspace of Ndim x
+// Ndim complex matrices: eleven at Ndim 25..256, none up to 8, eight at the
+// others) taken from the fixed array below instead of from device allocations.  The caller passes every input and output as device
 // memory it already owns.
 //
 // Properties of the fixed scratch:

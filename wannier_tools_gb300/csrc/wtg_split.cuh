@@ -26,9 +26,13 @@
 // `empty` barrier; no block-wide barrier separates chunks.  The first two
 // chunks of the next tile are generated before the accumulators of this one
 // are drained, so that the tensor cores restart at once after the drain.  What
-// bounds it: the MMA reads (A planes once per group of slice pairs, B planes
-// once) and the digit stores share the 128 B / clk of shared memory with the
-// tensor pipe at 60-80 %.
+// bounds it: the integer pipe.  At Ndim 112 (F16 digits) a chunk's digit planes
+// take 2.8 k cycles against 1.9 k of its MMAs, and 32 columns of accumulators
+// 11 k to read back, assemble and store; a product is 144 k cycles (28 chunks,
+// 4 tiles; 155 k with the residual's epilogue, 162 k with two FP64 sums).
+// Copying the A planes of the first column pass to global memory and loading
+// them for the others (bulk copies, 57 KB a chunk) was 5 % slower: they come back
+// no faster than they are made.
 //
 // Digits are made from packed integer extraction and one packed 16-bit
 // floating-point FMA per two digits (a digit's bits under a fixed exponent,
