@@ -887,112 +887,113 @@ __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, 
   int* const cL = (last && STACK && oL >= 3 && oL != 6 && oL != 7 && rb0 + quad * 32 + 31 >= N) ? s.cols(oL, N) : nullptr;
   unsigned rmax = 0;                       // upper words without sign: ordered like exponents
   const uint32_t tq = s.t().tslot + ((uint32_t)(quad * 32) << 16);
-  for (int cg = hw * 4; cg < width; cg += 16) {
+  // two columns at a time: the four warps of a quadrant share any pass width evenly (in
+  // fours, 24 and 40 columns took two and three rounds of four instead of 1.5 and 2.5:
+  // a product at Ndim 40 took 33.8 k cycles instead of 32.4)
 #pragma unroll 1
-    for (int c0 = cg; c0 < cg + 4; c0 += 2) {
-      uint32_t v[2][NACC][2];
-      uint32_t ta = tq + (uint32_t)c0;
+  for (int c0 = hw * 2; c0 < width; c0 += 8) {
+    uint32_t v[2][NACC][2];
+    uint32_t ta = tq + (uint32_t)c0;
 #pragma unroll
-      for (int a = 0; a < NACC; ++a)
+    for (int a = 0; a < NACC; ++a)
 #pragma unroll
-        for (int comp = 0; comp < 2; ++comp) {
-          tmem_ld2(ta, v[comp][a]);
-          ta += (uint32_t)width;
-        }
-      const int j0 = jb + c0;
-      const bool on0 = live && j0 < N, on1 = live && j0 + 1 < N;
-      double2* const p0 = o0b + (size_t)j0 * N;
-      double2* const q0 = o1b + (size_t)j0 * N;
-      double2 old0[2], old1[2];                 // the epilogue's loads
-      old0[0] = old0[1] = old1[0] = old1[1] = make_double2(0.0, 0.0);
-      if (epi == OZ_ADD2 || epi == OZ_ADDTO) {
-        if (on0) old1[0] = q0[0];
-        if (on1) old1[1] = q0[N];
+      for (int comp = 0; comp < 2; ++comp) {
+        tmem_ld2(ta, v[comp][a]);
+        ta += (uint32_t)width;
       }
-      if (epi == OZ_ADD2 || !first) {
-        if (on0) old0[0] = p0[0];
-        if (on1) old0[1] = p0[N];
+    const int j0 = jb + c0;
+    const bool on0 = live && j0 < N, on1 = live && j0 + 1 < N;
+    double2* const p0 = o0b + (size_t)j0 * N;
+    double2* const q0 = o1b + (size_t)j0 * N;
+    double2 old0[2], old1[2];                 // the epilogue's loads
+    old0[0] = old0[1] = old1[0] = old1[1] = make_double2(0.0, 0.0);
+    if (epi == OZ_ADD2 || epi == OZ_ADDTO) {
+      if (on0) old1[0] = q0[0];
+      if (on1) old1[1] = q0[N];
+    }
+    if (epi == OZ_ADD2 || !first) {
+      if (on0) old0[0] = p0[0];
+      if (on1) old0[1] = p0[N];
+    }
+    tmem_wait_ld();
+    double2 val[2];
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {          // without branches: four values in flight
+      const int ee = er + eY[min(j0 + jj, N - 1)];
+      uint32_t ar[NACC], ai[NACC];
+#pragma unroll
+      for (int a = 0; a < NACC; ++a) {
+        ar[a] = v[0][a][jj];
+        ai[a] = v[1][a][jj];
       }
-      tmem_wait_ld();
-      double2 val[2];
+      val[jj] = make_double2(K::value(ar, ee), K::value(ai, ee));
+    }
+    if (K::POISON) {
 #pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {          // without branches: four values in flight
-        const int ee = er + eY[min(j0 + jj, N - 1)];
-        uint32_t ar[NACC], ai[NACC];
-#pragma unroll
-        for (int a = 0; a < NACC; ++a) {
-          ar[a] = v[0][a][jj];
-          ai[a] = v[1][a][jj];
+      for (int jj = 0; jj < 2; ++jj)
+        if (max(er, eY[min(j0 + jj, N - 1)]) == 2047) {
+          val[jj].x = __longlong_as_double(0x7FF8000000000000LL);
+          val[jj].y = val[jj].x;
         }
-        val[jj] = make_double2(K::value(ar, ee), K::value(ai, ee));
-      }
-      if (K::POISON) {
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj)
-          if (max(er, eY[min(j0 + jj, N - 1)]) == 2047) {
-            val[jj].x = __longlong_as_double(0x7FF8000000000000LL);
-            val[jj].y = val[jj].x;
-          }
-      }
-      if (epi == OZ_ADD2) {
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          old1[jj].x += val[jj].x;
-          old1[jj].y += val[jj].y;
-          val[jj].x += old0[jj].x;
-          val[jj].y += old0[jj].y;
-        }
-        if (on0) q0[0] = old1[0];
-        if (on1) q0[N] = old1[1];
-      } else if (epi == OZ_IMINUS) {
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          if (first) {
-            val[jj] = make_double2(-val[jj].x, -val[jj].y);
-            // (one of the warp's rows is on the diagonal; FP64 adds are not free: two a clock)
-            if ((unsigned)(j0 + jj - rb0 - quad * 32) < 32u && rowL == j0 + jj)
-              val[jj].x = dsub_here(val[jj].x, -1.0);
-          } else {
-            val[jj] = make_double2(dsub_here(old0[jj].x, val[jj].x), dsub_here(old0[jj].y, val[jj].y));
-          }
-        }
-      } else if (epi == OZ_ADDTO || !first) {
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          const double2 o = first ? old1[jj] : old0[jj];
-          val[jj].x += o.x;
-          val[jj].y += o.y;
-        }
-      }
-      if (on0) p0[0] = val[0];
-      if (on1) p0[N] = val[1];
-      if (last && (epi == OZ_STORE_NORM || epi == OZ_IMINUS)) {
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          if (!(jj ? on1 : on0)) continue;
-          const float fr = upper_f32(val[jj].x), fi = upper_f32(val[jj].y);
-          if (K::FRO && epi == OZ_IMINUS) nrm = fmaf(fr, fr, fmaf(fi, fi, nrm));
-          else nrm += fr + fi;
-        }
-      }
-      unsigned e[2];
+    }
+    if (epi == OZ_ADD2) {
 #pragma unroll
       for (int jj = 0; jj < 2; ++jj) {
-        e[jj] = max((unsigned)__double2hiint(val[jj].x) & 0x7FFFFFFFu,
-                    (unsigned)__double2hiint(val[jj].y) & 0x7FFFFFFFu);
-        if (!(jj ? on1 : on0)) e[jj] = 0;
-        rmax = max(rmax, e[jj]);
+        old1[jj].x += val[jj].x;
+        old1[jj].y += val[jj].y;
+        val[jj].x += old0[jj].x;
+        val[jj].y += old0[jj].y;
       }
-      if (cU) {
-        const unsigned m0 = __reduce_max_sync(0xffffffffu, upper ? e[0] : 0u);
-        const unsigned m1 = __reduce_max_sync(0xffffffffu, upper ? e[1] : 0u);
-        if (lane < 2 && j0 + lane < N) atomicMax(&cU[j0 + lane], (int)((lane ? m1 : m0) >> 20));
+      if (on0) q0[0] = old1[0];
+      if (on1) q0[N] = old1[1];
+    } else if (epi == OZ_IMINUS) {
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        if (first) {
+          val[jj] = make_double2(-val[jj].x, -val[jj].y);
+          // (one of the warp's rows is on the diagonal; FP64 adds are not free: two a clock)
+          if ((unsigned)(j0 + jj - rb0 - quad * 32) < 32u && rowL == j0 + jj)
+            val[jj].x = dsub_here(val[jj].x, -1.0);
+        } else {
+          val[jj] = make_double2(dsub_here(old0[jj].x, val[jj].x), dsub_here(old0[jj].y, val[jj].y));
+        }
       }
-      if (cL) {
-        const unsigned m0 = __reduce_max_sync(0xffffffffu, upper ? 0u : e[0]);
-        const unsigned m1 = __reduce_max_sync(0xffffffffu, upper ? 0u : e[1]);
-        if (lane < 2 && j0 + lane < N) atomicMax(&cL[j0 + lane], (int)((lane ? m1 : m0) >> 20));
+    } else if (epi == OZ_ADDTO || !first) {
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        const double2 o = first ? old1[jj] : old0[jj];
+        val[jj].x += o.x;
+        val[jj].y += o.y;
       }
+    }
+    if (on0) p0[0] = val[0];
+    if (on1) p0[N] = val[1];
+    if (last && (epi == OZ_STORE_NORM || epi == OZ_IMINUS)) {
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        if (!(jj ? on1 : on0)) continue;
+        const float fr = upper_f32(val[jj].x), fi = upper_f32(val[jj].y);
+        if (K::FRO && epi == OZ_IMINUS) nrm = fmaf(fr, fr, fmaf(fi, fi, nrm));
+        else nrm += fr + fi;
+      }
+    }
+    unsigned e[2];
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {
+      e[jj] = max((unsigned)__double2hiint(val[jj].x) & 0x7FFFFFFFu,
+                  (unsigned)__double2hiint(val[jj].y) & 0x7FFFFFFFu);
+      if (!(jj ? on1 : on0)) e[jj] = 0;
+      rmax = max(rmax, e[jj]);
+    }
+    if (cU) {
+      const unsigned m0 = __reduce_max_sync(0xffffffffu, upper ? e[0] : 0u);
+      const unsigned m1 = __reduce_max_sync(0xffffffffu, upper ? e[1] : 0u);
+      if (lane < 2 && j0 + lane < N) atomicMax(&cU[j0 + lane], (int)((lane ? m1 : m0) >> 20));
+    }
+    if (cL) {
+      const unsigned m0 = __reduce_max_sync(0xffffffffu, upper ? 0u : e[0]);
+      const unsigned m1 = __reduce_max_sync(0xffffffffu, upper ? 0u : e[1]);
+      if (lane < 2 && j0 + lane < N) atomicMax(&cL[j0 + lane], (int)((lane ? m1 : m0) >> 20));
     }
   }
   if (last && ox >= 3 && live) atomicMax(&s.rows(ox, N)[rowL], (int)(rmax >> 20));
