@@ -28,8 +28,8 @@
 // are drained, so that the tensor cores restart at once after the drain.  What
 // bounds it: the integer pipe.  At Ndim 112 (F16 digits) a chunk's digit planes
 // take 2.8 k cycles against 1.9 k of its MMAs, and 32 columns of accumulators
-// 11 k to read back, assemble and store; a product is 144 k cycles (28 chunks,
-// 4 tiles; 155 k with the residual's epilogue, 162 k with two FP64 sums).
+// 11 k to read back, assemble and store; a product is 142 k cycles (28 chunks,
+// 4 tiles; 154 k with the residual's epilogue, 160 k with two FP64 sums).
 // Copying the A planes of the first column pass to global memory and loading
 // them for the others (bulk copies, 57 KB a chunk) was 5 % slower: they come back
 // no faster than they are made.
