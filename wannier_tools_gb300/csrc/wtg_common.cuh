@@ -117,7 +117,7 @@ struct DecimArgs {
   double2* gll;               // optional full outputs [n_inst][N*N] (null = skip)
   double2* grr;
   double2* gb;
-  double2* ws;                // [grid][8 or 9][N*N] workspace (decim_fp64_ws_matrices)
+  double2* ws;                // [grid][decim_fp64_ws_matrices(cfg)][N*N] workspace
   int* counter;               // work counter, zero at launch
   int KC;                     // GEMM k-chunk staged in shared memory
   int w0;                     // mixed: output-column pass width (tile table; 0 = built-in)
@@ -206,8 +206,8 @@ void tile_store(int precision, int N, int value);
 int decim_fp64_max_n();
 // Largest Ndim of the FP64 kernel whose inverse runs in global memory (above decim_fp64_max_n).
 int decim_fp64_large_max_n();
-// N x N complex workspace matrices per CTA of the FP64 kernel in this configuration (8, or 9
-// when the inverse runs in global memory).
+// N x N complex workspace matrices per CTA of the FP64 form in this configuration: 11 in the
+// split range, none for the warp-sized kernel, else 8, or 9 when the inverse runs in global memory.
 size_t decim_fp64_ws_matrices(const DecimConfig& cfg);
 // Launch shape for a given N on the current device (threads override: 0 = auto).  The inverse
 // runs in global memory above decim_fp64_max_n(), or at any N with force_global (the two
