@@ -1200,7 +1200,7 @@ __device__ __forceinline__ void gj_pivot_publish(const unsigned long long (&x)[R
   const unsigned pmin = __reduce_min_sync(0xffffffffu, cand ? (unsigned)bpos : 0xffffffffu);
   if (cand && (unsigned)bpos == pmin) {   // one lane: positions are distinct
     const int brow = lane + 32 * bm;
-    prow[t] = brow;
+    prow[t] = kmax == 1u ? -1 : brow;
     row_at[bpos] = rk;
     pos_of[rk] = bpos;
     row_at[t] = brow;
@@ -1361,9 +1361,10 @@ __device__ __noinline__ int gj32_start(const double2* __restrict__ X, double2 w,
     if (warp == 0) publish(0);
     gj_panel_sync();
     for (int t = 0; t < pb; ++t) {
-      if (misc[2 + b]) break;
+      const int p = prow[k0 + t];
+      if (p < 0) break;
       if (warp < pb) {
-        gj_step_cols<R, 1>(xp, cm + t * N, N, prow[k0 + t], rc[t], warp == t ? 0 : -1);
+        gj_step_cols<R, 1>(xp, cm + t * N, N, p, rc[t], warp == t ? 0 : -1);
         if (warp == t + 1) publish(t + 1);
       }
       gj_panel_sync();
@@ -1524,9 +1525,10 @@ __device__ __noinline__ int gj32_global(const double2* __restrict__ X, double2 w
       if (warp == 0) publish(0);
       __syncthreads();
       for (int t = 0; t < pb; ++t) {
-        if (misc[1]) break;
+        const int p = prow[k0 + t];
+        if (p < 0) break;
         if (warp < pb) {
-          gj_step_cols<R, 1>(xp, Cm + t * N, N, prow[k0 + t], recip[t], warp == t ? 0 : -1);
+          gj_step_cols<R, 1>(xp, Cm + t * N, N, p, recip[t], warp == t ? 0 : -1);
           if (warp == t + 1) publish(t + 1);
         }
         __syncthreads();
