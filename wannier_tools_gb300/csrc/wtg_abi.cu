@@ -388,8 +388,10 @@ int engine_create(int nmodels, const wtg_model_t* models, int precision, int max
     delete e;
     return cuda_fail(ce, "batch config");
   }
-  e->ph_off = (e->cfg.smem + 15) & ~(size_t)15;
-  e->cfg.smem = e->ph_off + ph_bytes;
+  if (ph_bytes > e->cfg.ph_room) {
+    e->ph_off = (e->cfg.smem + 15) & ~(size_t)15;
+    e->cfg.smem = e->ph_off + ph_bytes;
+  }
   int optin = 0, nsm = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

@@ -168,7 +168,8 @@ struct BatchArgs {
   int KC;                     // FP64 GEMM k-chunk
   int smem_gj_max;            // FP64 pipe kernel: largest Ndim whose inverse runs in shared memory
   int wb;                     // split products: B-plane width of the shared-memory layout
-  size_t ph_off;              // byte offset of the phase table (max nRu double2) in shared memory
+  size_t ph_off;              // byte offset of the phase table (max nRu double2) in shared memory:
+                              // behind the layout, or 0 where it fits DecimConfig::ph_room
 };
 
 struct DecimConfig {
@@ -181,6 +182,8 @@ struct DecimConfig {
   int w0 = 0;                 // mixed: output-column pass width
   int small = 0;              // FP64: lanes of a warp per instance, no workspace
   int split = 0;              // products on the tensor cores (mixed form; FP64 form's split kernel)
+  size_t ph_room = 0;         // FP64 batch: bytes at the start of shared memory that are free
+                              // until a point's Fourier sum is done (split products: the stages)
 };
 
 // Built-in choices and limits of the tunable shapes, and the mixed form's pass
@@ -245,8 +248,8 @@ cudaError_t launch_batch_split64(const BatchArgs& a, const DecimConfig& cfg, int
                                  cudaStream_t s);
 
 // Uneven batch launch shapes and launches.  The configs' shared memory excludes the
-// phase table, which the caller appends at BatchArgs::ph_off and adds to cfg.smem before
-// launching; extra_smem reserves room for it.
+// phase table (extra_smem bytes): it shares the first ph_room bytes, or the caller appends
+// it at BatchArgs::ph_off and adds it to cfg.smem before launching.
 cudaError_t batch_fp64_config(int max_n, size_t extra_smem, int* smem_gj_max, int* wb,
                               DecimConfig* cfg);
 cudaError_t launch_batch_fp64(const BatchArgs& a, const DecimConfig& cfg, int grid, cudaStream_t s);

@@ -322,9 +322,13 @@ static size_t batch_fp64_smem(int max_n, int max_smem_gj_n, int KC) {
 
 cudaError_t batch_fp64_config(int max_n, size_t extra_smem, int* smem_gj_max, int* wb,
                               DecimConfig* cfg) {
+  // the split kernel wherever the phase table fits its stages (206 KB: 12 864 R vectors); more
+  // take the FP64 pipe, whose shared memory leaves room for a few hundred to 1 300 others
   if (max_n >= FP64_SPLIT_MIN_N) {
     *smem_gj_max = 0;
-    return batch_split64_config(max_n, wb, cfg);
+    const cudaError_t e = batch_split64_config(max_n, wb, cfg);
+    if (e != cudaSuccess || extra_smem <= cfg->ph_room) return e;
+    *cfg = DecimConfig();
   }
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);

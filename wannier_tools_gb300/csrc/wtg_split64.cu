@@ -285,6 +285,7 @@ cudaError_t batch_split64_config(int max_n, int* wb, DecimConfig* cfg) {
   cfg->RP = 0;
   cfg->split = 1;
   cfg->smem = s64_smem(w);
+  cfg->ph_room = planes_bytes_of(w);
   cfg->ctas_per_sm = 1;
   return cudaSuccess;
 }
