@@ -219,6 +219,38 @@ __global__ void __launch_bounds__(SP_T, 1) k_batch_split64(const __grid_constant
   mx_teardown(s);
 }
 
+// Whether a split product X Y (workspace matrices 0 and 1 with their exponents) is as
+// accurate as an FP64 one in every element.  Its operands are rounded against their
+// row's (X) or column's (Y) maximum, so an element's error is K 2^-55 2^(er_i + ec_j)
+// whatever its terms are, an FP64 product's K 2^-53 sum_k |x_ik y_kj|.  With operands
+// graded along k (X D, D^-1 Y), or with sparse ones, the terms can lie far below the
+// product of the maxima (at n = 40, scales of 1e+-4 lose 2e-10 of the product, 1e+-8
+// all of it).  Required: sum_k |x_ik y_kj| >= 2^(er_i + ec_j), summed from exponents
+// alone, at most 4 times too small; an element without terms is an exact zero.  (Normal
+// random operands: at least 2.5 at n = 25, growing with n.)  Infinities and NaN fail:
+// a split product makes NaN of their whole row or column.  All threads.
+__device__ __noinline__ bool terms_reach_scales(const double2* W, int N, MxShared s) {
+  const double2* const X = W;
+  const double2* const Y = W + (size_t)N * N;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  bool low = false;
+  for (int j = warp; j < N; j += SP_T / 32) {
+    const int ec = s.cols(1, N)[j];
+    for (int i = lane; i < N; i += 32) {
+      const int er = s.rows(0, N)[i];
+      float sum = 0.f;
+      for (int k = 0; k < N; ++k) {
+        const double2 x = X[i + (size_t)k * N], y = Y[k + (size_t)j * N];
+        const bool none = (x.x == 0.0 && x.y == 0.0) || (y.x == 0.0 && y.y == 0.0);
+        const int e = max(bexp(x.x), bexp(x.y)) - er + max(bexp(y.x), bexp(y.y)) - ec;
+        if (!none) sum += __int_as_float((max(e, -100) + 127) << 23);      // e <= 0
+      }
+      low = low || (sum > 0.f && sum < 1.f) || max(er, ec) == 2047;
+    }
+  }
+  return !__syncthreads_or(low);
+}
+
 // one product (op 0) or inverse (op 1) by one CTA: W holds X, Y, the result and
 // five work matrices
 __global__ void __launch_bounds__(SP_T, 1) k_split64_unit(int op, int N, double2* W, int* status) {
@@ -231,7 +263,12 @@ __global__ void __launch_bounds__(SP_T, 1) k_split64_unit(int op, int N, double2
   if (op == 0) {
     exps_of(W, 0, N, s);
     exps_of(W + NN, 1, N, s);
-    f8_gemm7(W, ops(0, 1, 2), OZ_STORE, -1, pl, s);
+    if (terms_reach_scales(W, N, s)) {
+      f8_gemm7(W, ops(0, 1, 2), OZ_STORE, -1, pl, s);
+    } else {                                    // the FP64 pipe; its stages alias the split ones
+      const Shared f = fp64_layout(MxShared::base(), N, GJ_PANEL, false);
+      cta_gemm<13, EPI_STORE>(W, W + NN, N, GJ_PANEL, f.sX, f.sY, W + 2 * (size_t)NN, nullptr);
+    }
   } else {
     // C = X^-1: X given directly, so pass -X with w = 0 (M = 0*I - (-X) = X)
     double2* negX = W + 7 * (size_t)NN;
