@@ -251,6 +251,34 @@ __device__ __noinline__ bool terms_reach_scales(const double2* W, int N, MxShare
   return !__syncthreads_or(low);
 }
 
+// Whether the split residual I - X G (workspace matrices 0 and iG, both with their
+// exponents) resolves what an inverse of X owes: its rounding, 2^-55 2^(er_i + ec_j), is
+// to stay within 2^5 of the largest term x_ik g_kj a row has, taking G's largest column.
+// Graded columns of X put its terms far below: scales of 1e+-2 to 1e+-3 still meet the
+// residual's limit and left 1e-12 to 5e-10 in the rows of G, where an FP64 elimination
+// has 1e-14.  Up to 5 bits the split inverse is the closer one (random, row-graded and
+// ill-conditioned X: 0 to 2 bits).  All threads.
+__device__ __noinline__ bool residual_resolves(const double2* X, int iG, int N, MxShared s) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int* const top = s.t().prow;                       // per row: exponent of its largest term
+  for (int i = threadIdx.x; i < N; i += SP_T) top[i] = 0;
+  __syncthreads();
+  for (int k = warp; k < N; k += SP_T / 32) {
+    const int eg = s.rows(iG, N)[k];
+    for (int i = lane; i < N; i += 32) {
+      const double2 x = X[i + (size_t)k * N];
+      if (x.x != 0.0 || x.y != 0.0) atomicMax(&top[i], max(bexp(x.x), bexp(x.y)) + eg);
+    }
+  }
+  __syncthreads();
+  int ec = 0;
+  for (int j = lane; j < N; j += 32) ec = max(ec, s.cols(iG, N)[j]);
+  ec = __reduce_max_sync(0xffffffffu, ec);
+  bool low = false;
+  for (int i = threadIdx.x; i < N; i += SP_T) low = low || s.rows(0, N)[i] + ec > top[i] + 5;
+  return !__syncthreads_or(low);
+}
+
 // one product (op 0) or inverse (op 1) by one CTA: W holds X, Y, the result and
 // five work matrices
 __global__ void __launch_bounds__(SP_T, 1) k_split64_unit(int op, int N, double2* W, int* status) {
@@ -277,6 +305,9 @@ __global__ void __launch_bounds__(SP_T, 1) k_split64_unit(int op, int N, double2
     int G = 3, Gn = 4;
     sing = s64_inverse(7, make_double2(0.0, 0.0), W, pl, G, Gn, 6, 5, -1, -1, 0, s);
     __syncthreads();
+    exps_of(W, 0, N, s);
+    if (!sing && !s.t().abort && !residual_resolves(W, G, N, s))
+      sing = gj64(negX, make_double2(0.0, 0.0), N, W + (size_t)G * NN, W + 6 * (size_t)NN, 0);
     double2* C = W + 2 * (size_t)NN;
     for (int e = tid; e < NN; e += blockDim.x) C[e] = W[(size_t)G * NN + e];
   }
