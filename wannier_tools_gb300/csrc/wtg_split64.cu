@@ -36,9 +36,95 @@ namespace {
 #include "wtg_fp64_solve.cuh"
 #include "wtg_small_dev.cuh"
 
-// Decimation of one instance whose eps, eps_s, eps_t (= H00), alpha (= H01) and
-// beta (= H01^dagger) already sit in workspace matrices 0..4 of W (11 N x N
-// matrices), as fp64_solve; all threads.
+// Whether a point may run on split products: operands rounded against their row's or
+// column's maximum (2^-55 of it, for real and imaginary parts together) lose what an
+// FP64 product keeps
+//   - where orbitals have very different scales (M = w - H00 and H01): an inner index of
+//     the products then joins large columns to small rows;
+//   - where eta is very small: off the bands the imaginary parts, which the spectral sums
+//     read, are about eta / |M| of the real ones.
+// The largest elements of the orbitals' rows and columns have to lie within a factor of
+// 2^6 and eta within 2^20 of the largest of all.  Relative errors of the sums, split
+// against FP64 arithmetic (emulated, Ndim 27..40, against 64-bit mantissas): scales within
+// 2^5 median 1e-13 and 1e-13, at 2^6 at most 3.4e-12 and 5.7e-12, at 2^9 4e-12 (worst
+// 6e-11) and 2e-13, on-site 1e12 beside hopping 1e6 5e-8 and 4e-13; energies 20 eV off the
+// bands at eta 1e-3 eV (2^-15) 3e-13 and 1e-14, 1e-6 eV 2e-10 and 1e-11, 1e-10 eV 5e-6 and
+// 1e-7 (a real H keeps 1e-16 in FP64).  One pass over H00 and H01 that also makes alpha's
+// exponents (as exps_of); E and Al are workspace matrices 0 and 3; all threads.
+__device__ __noinline__ bool split_suits(const double2* __restrict__ W, double2 w, int N, MxShared s) {
+  constexpr int Al = 3;
+  const double2* const A = W + (size_t)Al * N * N;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int* const top = s.t().prow;                      // exponent of an orbital's largest element
+  int* const er = s.rows(Al, N);
+  int* const ec = s.cols(Al, N);
+  for (int i = threadIdx.x; i < N; i += SP_T) {
+    er[i] = EXP_MIN;
+    top[i] = 0;
+  }
+  __syncthreads();
+  constexpr int ROWS = FP64_SPLIT_MAX_N / 32;
+  int amax[ROWS], tmax[ROWS];
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) amax[q] = tmax[q] = 0;
+  for (int j = warp; j < N; j += SP_T / 32) {
+    int ca = EXP_MIN, ct = 0;
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+      const int i = lane + 32 * q;
+      if (i < N) {
+        const double2 a = A[i + (size_t)j * N];
+        double2 m = W[i + (size_t)j * N];
+        if (i == j) m = make_double2(w.x - m.x, w.y - m.y);
+        const int ea = max(bexp(a.x), bexp(a.y)), et = max(ea, max(bexp(m.x), bexp(m.y)));
+        amax[q] = max(amax[q], ea);
+        tmax[q] = max(tmax[q], et);
+        ca = max(ca, ea);
+        ct = max(ct, et);
+      }
+    }
+    ca = __reduce_max_sync(0xffffffffu, ca);
+    ct = __reduce_max_sync(0xffffffffu, ct);
+    if (lane == 0) {
+      ec[j] = ca;
+      atomicMax(&top[j], ct);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    const int i = lane + 32 * q;
+    if (i < N) {
+      atomicMax(&er[i], amax[q]);
+      atomicMax(&top[i], tmax[q]);
+    }
+  }
+  __syncthreads();
+  int hi = 0, lo = 2047;
+  for (int i = lane; i < N; i += 32) {
+    hi = max(hi, top[i]);
+    lo = min(lo, top[i]);
+  }
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  __syncthreads();
+  // (infinities and NaN: no form has a result)
+  return hi == 2047 || (hi - lo <= 6 && hi - bexp(w.y) <= 20);
+}
+
+// a point on the FP64 pipe in the shared memory of the split products
+template <class O, class Emit>
+__device__ __forceinline__ void pipe_solve(int N, double2 w, const O& o, double2* gll, double2* grr,
+                                           double2* gb, double2* W, int gi, Emit emit) {
+  constexpr int KC = 16;
+  if (N <= MX_SMEM_GJ_N && !gi)
+    fp64_solve<13, false>(N, KC, w, o, gll, grr, gb, W, fp64_layout(MxShared::base(), N, KC, true), emit);
+  else
+    fp64_solve<13, true>(N, KC, w, o, gll, grr, gb, W, fp64_layout(MxShared::base(), N, KC, false), emit);
+}
+
+// Decimation of one instance whose eps, eps_s, eps_t (= H00), alpha (= H01, with
+// its exponents) and beta (= H01^dagger) already sit in workspace matrices 0..4 of
+// W (11 N x N matrices), as fp64_solve; all threads.
 template <class O, class Emit>
 __device__ __forceinline__ void s64_solve(const MxPlan& pl, double2 w, const O& o, double2* gll,
                                           double2* grr, double2* gb, double2* W, int gi,
@@ -49,7 +135,6 @@ __device__ __forceinline__ void s64_solve(const MxPlan& pl, double2 w, const O& 
   int stat = 0, it = 0;
   bool conv = false;
   split_tables<F8x7, F8x4>(pl, s);
-  exps_of(W + (size_t)Al * NN, Al, N, s);
   exps_dagger(Be, Al, N, s);
   for (int itc = 1; itc <= o.itermax && !s.t().abort; ++itc) {   // src/surfgreen.f90:86-122
     it = itc;
@@ -88,6 +173,30 @@ __device__ __forceinline__ void s64_solve(const MxPlan& pl, double2 w, const O& 
   __syncthreads();
 }
 
+// an instance's outputs
+__device__ __forceinline__ void put_point(const DecimArgs& a, int inst, double dl, double dr, double db,
+                                          const double* spin, int it, int stat) {
+  const size_t oidx = (size_t)(a.k_offset + inst / a.nomega) + (size_t)(inst % a.nomega) * a.nk_total;
+  a.dos_l[oidx] = dl;
+  a.dos_r[oidx] = dr;
+  a.dos_bulk[oidx] = db;
+  if (a.spin[0])
+    for (int c = 0; c < 6; ++c) a.spin[c][oidx] = spin[c];
+  if (a.iters) a.iters[oidx] = it;
+  if (a.status) a.status[oidx] = (uint8_t)stat;
+}
+
+// an instance that split products do not suit; a function of its own, so that the split
+// path shares no registers or stack with it (inlined, a product-bound point was 0.7 % slower)
+__device__ __noinline__ void pipe_point(const DecimArgs& a, int inst, double2* W, int gi) {
+  const size_t NN = (size_t)a.N * a.N;
+  pipe_solve(a.N, make_double2(a.omega[inst % a.nomega], a.eta), a, a.gll ? a.gll + inst * NN : nullptr,
+             a.grr ? a.grr + inst * NN : nullptr, a.gb ? a.gb + inst * NN : nullptr, W, gi,
+             [&](double dl, double dr, double db, const double* spin, int it, int stat) {
+               put_point(a, inst, dl, dr, db, spin, it, stat);
+             });
+}
+
 __global__ void __launch_bounds__(SP_T, 1) k_decimate_split64(const __grid_constant__ DecimArgs a,
                                                               int gi) {
   const int N = a.N, NN = N * N, T = blockDim.x, tid = threadIdx.x;
@@ -102,17 +211,11 @@ __global__ void __launch_bounds__(SP_T, 1) k_decimate_split64(const __grid_const
     __syncthreads();
     if (inst >= a.n_inst) break;
     const int ik = inst / a.nomega, iw = inst % a.nomega;
-    const size_t oidx = (size_t)(a.k_offset + ik) + (size_t)iw * a.nk_total;
     if (s.t().abort) {       // a wait gave up earlier: the rest of this CTA's points are not computed
       if (tid == 0) {
         const double nan = __longlong_as_double(0x7FF8000000000000LL);
-        a.dos_l[oidx] = nan;
-        a.dos_r[oidx] = nan;
-        a.dos_bulk[oidx] = nan;
-        if (a.spin[0])
-          for (int c = 0; c < 6; ++c) a.spin[c][oidx] = nan;
-        if (a.iters) a.iters[oidx] = 0;
-        if (a.status) a.status[oidx] = (uint8_t)PT_TIMEOUT;
+        const double spin[6] = {nan, nan, nan, nan, nan, nan};
+        put_point(a, inst, nan, nan, nan, spin, 0, PT_TIMEOUT);
       }
       continue;
     }
@@ -130,25 +233,23 @@ __global__ void __launch_bounds__(SP_T, 1) k_decimate_split64(const __grid_const
       W[4 * NN + j + (size_t)i * N] = make_double2(t.x, -t.y);
     }
     __syncthreads();
+    if (!split_suits(W, w, N, s)) {
+      pipe_point(a, inst, W, gi);
+      continue;
+    }
     s64_solve(pl, w, a, a.gll ? a.gll + (size_t)inst * NN : nullptr,
               a.grr ? a.grr + (size_t)inst * NN : nullptr,
               a.gb ? a.gb + (size_t)inst * NN : nullptr, W, gi, s,
               [&](double dl, double dr, double db, const double* spin, int it, int stat) {
-                a.dos_l[oidx] = dl;
-                a.dos_r[oidx] = dr;
-                a.dos_bulk[oidx] = db;
-                if (a.spin[0])
-                  for (int c = 0; c < 6; ++c) a.spin[c][oidx] = spin[c];
-                if (a.iters) a.iters[oidx] = it;
-                if (a.status) a.status[oidx] = (uint8_t)stat;
+                put_point(a, inst, dl, dr, db, spin, it, stat);
               });
   }
   mx_teardown(s);
 }
 
 // Uneven batch (several models, eta per point) in one persistent launch, as
-// k_batch_fp64 of wtg_decimate.cu: points outside the split range run on the FP64
-// pipe, the others as k_decimate_split64.
+// k_batch_fp64 of wtg_decimate.cu: points outside the split range, or that split
+// products do not suit, run on the FP64 pipe, the others as k_decimate_split64.
 __global__ void __launch_bounds__(SP_T, 1) k_batch_split64(const __grid_constant__ BatchArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
   const int tid = threadIdx.x;
@@ -200,16 +301,11 @@ __global__ void __launch_bounds__(SP_T, 1) k_batch_split64(const __grid_constant
       if (a.iters) a.iters[p] = it;
       if (a.status) a.status[p] = (uint8_t)st;
     };
-    constexpr int KC = 16;
     if (m.N <= SMALL_MAX_N) {                // one warp, as k_decimate_small
       if (tid < 32) small_point(m.N, w, o, W, emit);
       __syncthreads();
-    } else if (m.N > FP64_SPLIT_MAX_N) {
-      fp64_solve<13, true>(m.N, KC, w, o, nullptr, nullptr, nullptr, W,
-                           fp64_layout(smem_dyn, m.N, KC, false), emit);
-    } else if (m.N < FP64_SPLIT_MIN_N) {
-      fp64_solve<13, false>(m.N, KC, w, o, nullptr, nullptr, nullptr, W,
-                            fp64_layout(smem_dyn, m.N, KC, true), emit);
+    } else if (m.N < FP64_SPLIT_MIN_N || m.N > FP64_SPLIT_MAX_N || !split_suits(W, w, m.N, s)) {
+      pipe_solve(m.N, w, o, nullptr, nullptr, nullptr, W, 0, emit);
     } else {
       MxPlan pl = s64_plan(m.N);
       pl.wb = a.wb;
