@@ -379,8 +379,9 @@ int wtg_batch_spectrum(int nmodels, const wtg_model_t* models, int npts, const i
  *                                 Gauss-Jordan runs in global memory at every
  *                                 Ndim (the variant for large matrices; both
  *                                 agree bit for bit)
- *   WTG_TEST_MIXED_SPIN_LIMIT     > 0: the mixed kernels' pipeline waits on the
- *                                 tensor cores give up after this many
+ *   WTG_TEST_MIXED_SPIN_LIMIT     > 0: the pipeline waits on the tensor cores of
+ *                                 the mixed kernels and of the FP64 form's split
+ *                                 kernels (Ndim 25..256) give up after this many
  *                                 non-blocking polls instead of the built-in
  *                                 bound, so that a test can make them run out:
  *                                 the points get WTG_PT_TIMEOUT and the call

@@ -198,11 +198,11 @@ __device__ __noinline__ void pipe_point(const DecimArgs& a, int inst, double2* W
 }
 
 __global__ void __launch_bounds__(SP_T, 1) k_decimate_split64(const __grid_constant__ DecimArgs a,
-                                                              int gi) {
+                                                              int gi, unsigned spin_limit) {
   const int N = a.N, NN = N * N, T = blockDim.x, tid = threadIdx.x;
   const MxPlan pl = s64_plan(N);
   const MxShared s = mx_layout(pl.wb);
-  mx_setup(s, 0u);
+  mx_setup(s, spin_limit);
   double2* W = a.ws + (size_t)blockIdx.x * 11 * NN;
   for (;;) {
     if (tid == 0) s.t().misc[0] = atomicAdd(a.counter, 1);
@@ -250,11 +250,12 @@ __global__ void __launch_bounds__(SP_T, 1) k_decimate_split64(const __grid_const
 // Uneven batch (several models, eta per point) in one persistent launch, as
 // k_batch_fp64 of wtg_decimate.cu: points outside the split range, or that split
 // products do not suit, run on the FP64 pipe, the others as k_decimate_split64.
-__global__ void __launch_bounds__(SP_T, 1) k_batch_split64(const __grid_constant__ BatchArgs a) {
+__global__ void __launch_bounds__(SP_T, 1) k_batch_split64(const __grid_constant__ BatchArgs a,
+                                                           unsigned spin_limit) {
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
   const int tid = threadIdx.x;
   const MxShared s = mx_layout(a.wb);
-  mx_setup(s, 0u);
+  mx_setup(s, spin_limit);
   double2* W = a.ws + (size_t)blockIdx.x * a.ws_stride;
   const int npts = a.run ? a.run->npts : a.npts;
   const double tol = a.run ? a.run->tol : a.tol;
@@ -470,7 +471,8 @@ cudaError_t batch_split64_prepare() {
 
 cudaError_t launch_batch_split64(const BatchArgs& a, const DecimConfig& cfg, int grid,
                                  cudaStream_t s) {
-  k_batch_split64<<<grid, cfg.threads, cfg.smem, s>>>(a);
+  k_batch_split64<<<grid, cfg.threads, cfg.smem, s>>>(
+      a, (unsigned)test_option(WTG_TEST_MIXED_SPIN_LIMIT));
   return cudaGetLastError();
 }
 
@@ -484,7 +486,8 @@ cudaError_t launch_split64_unit(int op, int N, double2* W, int* status, cudaStre
 }
 
 cudaError_t launch_split64(const DecimArgs& a, const DecimConfig& cfg, int grid, cudaStream_t s) {
-  k_decimate_split64<<<grid, cfg.threads, cfg.smem, s>>>(a, cfg.inv_global);
+  k_decimate_split64<<<grid, cfg.threads, cfg.smem, s>>>(
+      a, cfg.inv_global, (unsigned)test_option(WTG_TEST_MIXED_SPIN_LIMIT));
   return cudaGetLastError();
 }
 
