@@ -194,11 +194,6 @@ size_t smem_bytes(int N, int KC, bool inv_in_smem) {
   return big * 16 + (size_t)N * 32 + 16 * GJ_PANEL + 32 * 8 + (size_t)N * 8 + 16;
 }
 
-template <int RP>
-const void* fp64_kernel(bool gi) {
-  return gi ? (const void*)k_decimate_fp64<13, true> : (const void*)k_decimate_fp64<RP, false>;
-}
-
 }  // namespace
 
 int decim_fp64_max_n() {
@@ -219,7 +214,7 @@ int fp64_threads_for(int N, long long n_inst, int nsm) {
   // point against 128 threads); with many, narrow ones keep more instances in
   // flight (20 000, 16 875 and 8 639 points: 38.6 -> 32.1, 43.5 -> 43.3, 52.5 ->
   // 46.7 ms with 64 threads)
-  if (N >= 12 && N <= 32 && n_inst <= nsm) return 256;
+  if (N >= 12 && n_inst <= nsm) return 256;
   if (N <= 20 && n_inst >= 8LL * nsm) return 64;
   return fp64_threads_default(N);
 }
@@ -228,7 +223,8 @@ size_t decim_fp64_ws_matrices(const DecimConfig& cfg) {
   return cfg.small ? 0 : cfg.split ? 11 : cfg.inv_global ? 9 : 8;
 }
 
-// launch shape of the kernel on the FP64 pipe
+// launch shape of the kernel on the FP64 pipe (Ndim 9..24, above 256 and in the unit
+// kernel; any with force_global)
 static cudaError_t dfma_config(int N, int threads_override, DecimConfig* cfg, bool force_global) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -240,26 +236,19 @@ static cudaError_t dfma_config(int N, int threads_override, DecimConfig* cfg, bo
   if (gi && N > decim_fp64_large_max_n()) return cudaErrorInvalidValue;
   if (threads_override <= 0) threads_override = tile_value(0, N);
   int T = threads_override > 0 ? threads_override : fp64_threads_default(N);
-  int KC = N;
-  if (gi) {
-    T = 256;                       // 255 registers: a lane keeps 10 rows of a column
-    KC = 16;
-  } else if (smem_bytes(N, KC, true) > (size_t)smem_optin) {
-    KC = (N + 1) / 2;
-  }
-  while (KC > GJ_PANEL && smem_bytes(N, KC, !gi) > (size_t)smem_optin) --KC;
+  if (gi) T = 256;                 // 255 registers: a lane keeps 10 rows of a column
+  const int KC = gi ? 16 : N;
   if (smem_bytes(N, KC, !gi) > (size_t)smem_optin) return cudaErrorInvalidValue;
-  const int rounds = (N * N + T - 1) / T;
-  int RP = 13;
-  if (!gi && rounds <= 4) RP = 4;
-  else if (!gi && rounds <= 8) RP = 8;
+  const int rounds = (N * N + T - 1) / T;      // at most 7 where not gi
+  const int RP = gi ? 13 : rounds <= 4 ? 4 : 8;
   cfg->threads = T;
   cfg->KC = KC;
   cfg->RP = RP;
   cfg->inv_global = gi ? 1 : 0;
   cfg->smem = smem_bytes(N, KC, !gi);
   int occ = 0;
-  const void* fn = RP == 4 ? fp64_kernel<4>(gi) : (RP == 8 ? fp64_kernel<8>(gi) : fp64_kernel<13>(gi));
+  const void* fn = gi ? (const void*)k_decimate_fp64<13, true>
+                   : RP == 4 ? (const void*)k_decimate_fp64<4, false> : (const void*)k_decimate_fp64<8, false>;
   e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg->smem);
   if (e != cudaSuccess) return e;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, T, cfg->smem);
@@ -297,15 +286,9 @@ cudaError_t launch_decimate_fp64(const DecimArgs& a, const DecimConfig& cfg, int
     else k_decimate_small<8><<<grid, cfg.threads, 0, s>>>(a);
     return cudaGetLastError();
   }
-  if (cfg.inv_global) {
-    k_decimate_fp64<13, true><<<grid, cfg.threads, cfg.smem, s>>>(a);
-    return cudaGetLastError();
-  }
-  switch (cfg.RP) {
-    case 4: k_decimate_fp64<4, false><<<grid, cfg.threads, cfg.smem, s>>>(a); break;
-    case 8: k_decimate_fp64<8, false><<<grid, cfg.threads, cfg.smem, s>>>(a); break;
-    default: k_decimate_fp64<13, false><<<grid, cfg.threads, cfg.smem, s>>>(a); break;
-  }
+  if (cfg.inv_global) k_decimate_fp64<13, true><<<grid, cfg.threads, cfg.smem, s>>>(a);
+  else if (cfg.RP == 4) k_decimate_fp64<4, false><<<grid, cfg.threads, cfg.smem, s>>>(a);
+  else k_decimate_fp64<8, false><<<grid, cfg.threads, cfg.smem, s>>>(a);
   return cudaGetLastError();
 }
 
