@@ -426,6 +426,8 @@ class SpectrumRun:
             peak = MEASURED_PEAKS.get("bf16_tflops")
             traffic = traffic_per_solve(self.wl_name(), "k_decimate_split64")
             return {"bound": "tensor", "kernel": "k_decimate_split64", "achieved": ach, "peak": peak,
+                    "limited_by": "digit generation and accumulator read-back taking turns on the "
+                                  "integer pipe (50 % of it), not the tensor pipe",
                     "unit": "TFLOP/s", "frac": (ach / peak) if (ach and peak) else None,
                     "traffic": (traffic * self.B * self.nomega) if traffic else None,
                     "traffic_unit": "bytes per launch",
@@ -455,6 +457,8 @@ class SpectrumRun:
         iss = issued / (prof["decim_ms"] / 1e3) / 1e12 if prof["decim_ms"] > 0 else None
         peak = MEASURED_PEAKS.get("bf16_tflops")
         return {"bound": "tensor", "kernel": "k_decimate_mixed", "achieved": ach, "peak": peak,
+                "limited_by": "digit generation and accumulator read-back taking turns on the "
+                              "integer pipe, not the tensor pipe",
                 "unit": "TFLOP/s", "frac": (ach / peak) if (ach and peak) else None, "traffic": None,
                 "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst)", "launch_ms": launch_ms,
                 "work": "(56*it+24)*Ndim^3 FP64-equivalent flops per solve (algorithmic)",

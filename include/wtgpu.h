@@ -59,12 +59,19 @@ extern "C" {
 
 /* precision modes */
 #define WTG_PREC_FP64  0        /* FP64 decimation; Ndim <= 320.  At Ndim 25..256 every product is
-                                   an exactly split product on the tcgen05 tensor cores (55-bit
-                                   operands in balanced 8-bit digits, exact integer accumulation,
-                                   smaller error than an FP64 product) and an inverse an FP32
-                                   Gauss-Jordan refined on such products to FP64's residual, or
-                                   the FP64 Gauss-Jordan where that does not converge (condition
-                                   beyond ~1e7); at other Ndim all on the FP64 pipe */
+                                   a split product on the tcgen05 tensor cores (operands rounded
+                                   to 2^-54 of their row's or column's leading digit, balanced
+                                   8-bit digits, integer accumulation): element (i, j) is within
+                                   about K 2^-51 of the scale 2^(er_i + ec_j) of its row and
+                                   column, below an FP64 product's error where its terms reach
+                                   that scale, and an inverse an FP32 Gauss-Jordan refined on
+                                   such products, or the FP64 Gauss-Jordan where that does not
+                                   converge (condition beyond ~1e7).  Points whose orbitals'
+                                   largest elements (of w - H00 and H01) differ by more than
+                                   2^6, or whose eta is below 2^-20 of the largest, run on the
+                                   FP64 pipe (as every point at other Ndim), 2-10 times slower;
+                                   wtg_mat_mul and wtg_inv take it where their operands' scales
+                                   differ along the contraction */
 #define WTG_PREC_MIXED 1        /* products as BF16 digit splits on the tcgen05 tensor cores
                                    (49-bit rounded operands in balanced 7-bit digits, FP32
                                    accumulation exact per slice order up to 6, int64
@@ -359,7 +366,9 @@ int wtg_engine_graph_info(wtg_engine_t engine, int* graphs, long long* graph_lau
  * the order of the convergence norm's block sum (every output element is summed in
  * the same order; spectra agree to 1e-12).  Set tiles before creating engines
  * (an engine keeps the widths it was created with); wtg_tile_get returns the
- * value in use and the built-in one.  No counterpart in the reference.
+ * value stored, or the built-in one, and the built-in one (FP64: that of the CTA-wide
+ * kernel; at Ndim 9..24 it is 64 or 256 for very many or few instances).  No
+ * counterpart in the reference.
  */
 int wtg_tile_set(int precision, int ndim, int value);
 int wtg_tile_get(int precision, int ndim, int* value, int* builtin);

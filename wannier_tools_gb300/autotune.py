@@ -2,8 +2,10 @@
 
 The tunable shape is, per Ndim,
 
-* FP64 (per-model kernel, Ndim <= 119 where the inverse runs in shared memory):
-  threads per CTA, 128, 256 or 512 (the GEMM's register rows per pass follow);
+* FP64: threads per CTA of the CTA-wide kernel, 128, 256 or 512 (the GEMM's register
+  rows per pass follow).  It runs at Ndim 9..24, where a stored value replaces the
+  built-in choice by instance count; at the other candidates' sizes (up to 8, 25..119)
+  other kernels run and every value gives the same launch;
 * mixed (split-BF16 products on the tensor cores): the output-column pass width,
   a multiple of 8 up to the tensor-memory limit (40 columns: 2 x 6 accumulators
   of w columns in 512), i.e. how many passes of 2 x nacc accumulators cover the product.
@@ -31,7 +33,7 @@ import numpy as np
 
 TABLE = Path(__file__).resolve().with_name("tiles.json")
 FORMS = {"fp64": 0, "mixed": 1}
-FP64_SMEM_INVERSE_MAX_N = 119   # above this the FP64 kernel's inverse runs in global memory (256 threads)
+FP64_SMEM_INVERSE_MAX_N = 119   # above this a CTA-wide FP64 inverse runs in global memory (256 threads)
 MIXED_MAX_N = 320
 
 

@@ -15,8 +15,8 @@
 //          other, which truncates at about 2^-51 of the result)
 //   DigF8  55-bit operands (rounded to nearest) in seven base-256 digits as
 //          F16; orders 2..9, one exact accumulator each, so a product is as
-//          accurate as the rounding of its operands (DigF8<4>: the leading
-//          four digits and orders 2..5)
+//          accurate as the rounding of its operands against those exponents
+//          (DigF8<4>: the leading four digits and orders 2..5)
 //
 // Pipeline of one product (split_gemm).  The tiles of the product (row block x
 // column pass) are cut into K chunks of 16; the chunks of all tiles form one
@@ -26,7 +26,9 @@
 // `empty` barrier; no block-wide barrier separates chunks.  The first two
 // chunks of the next tile are generated before the accumulators of this one
 // are drained, so that the tensor cores restart at once after the drain.  What
-// bounds it: the integer pipe.  At Ndim 112 (F16 digits) a chunk's digit planes
+// bounds it: the two integer-heavy phases, which take turns at one CTA an SM (the
+// pipe is 65-70 % busy in them, 50 % over a launch, and so are the issue slots;
+// profiles/k_decimate_split64_arc_n112.md).  At Ndim 112 (F16 digits) a chunk's digit planes
 // take 2.8 k cycles against 1.9 k of its MMAs, and 32 columns of accumulators
 // 11 k to read back, assemble and store; a product is 142 k cycles (28 chunks,
 // 4 tiles; 154 k with the residual's epilogue, 160 k with two FP64 sums).
@@ -36,8 +38,8 @@
 //
 // Digits are made from packed integer extraction and one packed 16-bit
 // floating-point FMA per two digits (a digit's bits under a fixed exponent,
-// minus the offset: exact).  Generation and drain are bound by the integer pipe
-// (64 lanes a clock per SM), so both are written for few integer instructions.
+// minus the offset: exact).  Generation and drain are mostly integer instructions
+// (64 lanes a clock per SM), so both are written for few of them.
 //
 // Every mbarrier wait is bounded; on a timeout the CTA stops issuing work,
 // marks the instance, waits (bounded) for its MMAs and frees tensor memory.
@@ -856,7 +858,7 @@ __device__ __forceinline__ float upper_f32(double x) {
 }
 
 // Accumulators of a tile through the epilogue (all warps: four per quadrant of
-// 32 tensor-memory lanes, each taking 4 of every 16 columns).  Returns this
+// 32 tensor-memory lanes, each taking 2 of every 8 columns).  Returns this
 // thread's part of the product's FP32 sum.
 template <class K>
 __device__ __noinline__ float split_drain(double2* __restrict__ W, uint32_t op, int EPI, int EPI2,

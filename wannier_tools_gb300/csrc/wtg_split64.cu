@@ -8,10 +8,12 @@
 // src/mat_mul.f90:23) is an exactly split product (split_gemm of wtg_split.cuh
 // with DigF8 digits): 55-bit operands against a shared exponent per row /
 // column, seven base-256 digits, the slice orders 2..9 in one exact integer
-// accumulator each.  Its error (operand rounding, 2^-55 of the row or column
-// maximum) is below that of an FP64 product, whose partial sums round K times:
-// against exact products of normal random complex matrices it is 3-6 times
-// smaller at Ndim 40..320.
+// accumulator each.  Its error is the operands' rounding against their row's or
+// column's maximum, real and imaginary parts together: below an FP64 product's,
+// whose partial sums round K times, where the terms reach those maxima (against
+// exact products of normal random complex matrices 3-6 times smaller at Ndim
+// 40..320), above it for operands graded along k and for imaginary parts far below
+// the real ones.  Points of that kind run on the FP64 pipe (split_suits).
 //
 // Inverses (zgesv with identity, src/inverse.f90:43-55): an FP32 Gauss-Jordan
 // with partial pivoting gives a starting point, and Newton-Schulz steps
